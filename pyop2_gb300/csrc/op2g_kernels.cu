@@ -56,7 +56,10 @@ struct SpDev {
 
 __device__ __forceinline__ bool vcell(const SpDev &S, const PairDev &P, long long v,
                                       long long &rent, long long &cent, int &layer, int &nl) {
-    const long long e = S.extruded ? v / S.slots : v;
+    // (a 64-bit division costs several times a 32-bit one)
+    const long long e = !S.extruded ? v
+                        : v >> 32   ? v / S.slots
+                                    : (long long)((unsigned)v / (unsigned)S.slots);
     const int l = S.extruded ? (int)(v - e * S.slots) : 0;
     rent = e;
     cent = e;
@@ -85,7 +88,9 @@ __device__ __forceinline__ bool vcell(const SpDev &S, const PairDev &P, long lon
 
 __device__ __forceinline__ int ext_term(int layer, int k, int q, int nl) {
     const int eff = layer + k + q;
-    return nl > 0 ? (eff % nl - q % nl) : (eff - q);
+    if (nl <= 0) return eff - q;
+    // the remainders are taken only where they change the value
+    return (eff < nl ? eff : eff % nl) - (q < nl ? q : q % nl);
 }
 
 // Row (column) of local entry ir (jr) of facet k of a virtual cell: the
@@ -104,43 +109,516 @@ __device__ __forceinline__ int col_of(const SpDev &S, const PairDev &P, long lon
     return b;
 }
 
-// Row -> virtual-cell incidence: counts (pass 0) or fills (pass 1).
-// With a single pair every incidence brings the same number of candidate
-// columns (tc), so the candidate counts follow from the incidence counts
-// and cand is left untouched (one atomic per incidence instead of two).
-// narrow: the transpose list holds 32-bit entity numbers (one pair over a
-// flat set), otherwise 64-bit codes (pair << 56 | virtual cell).
-__global__ void k_incidence(SpDev S, const PairDev *__restrict__ pairs, int p, int pass,
-                            int single_pair, int narrow, long long *__restrict__ cnt,
-                            int *__restrict__ cand, int *__restrict__ fillpos,
-                            long long *__restrict__ tlist) {
+// What an entry of the row -> virtual-cell transpose list holds:
+enum {
+    E_CODE = 0,   // 64 bits, pair << 56 | virtual cell: several pairs, composed
+                  // maps or per-entity layers
+    E_FLAT = 1,   // 32 bits, the entity: one pair over a flat set
+    E_LAYER = 2,  // 64 bits, entity << 32 | layer: one pair over a set with the
+                  // same layers everywhere, so that reading an entry back takes
+                  // no division and no load of the layers
+};
+
+// Row -> virtual-cell incidence: counts into cnt (pass 0), or fills the list
+// (pass 1, ptr = the scanned counts; cnt counts down to zero again).  When all
+// pairs bring the same number of candidate columns (tc) the candidate counts
+// follow from the incidence counts and cand is NULL.
+//
+// Bound by the atomics on the row counters: a cell's are issued four at a
+// time before any result is used, and lanes next to each other that name the
+// same row (on a mesh numbered cell by cell, the vertices that neighbouring
+// cells share) count together, one atomic for the run.
+template <int EMODE>
+__global__ void __launch_bounds__(256)
+    k_incidence(SpDev S, const PairDev *__restrict__ pairs, int p, int pass,
+                int *__restrict__ cnt, int *__restrict__ cand,
+                const long long *__restrict__ ptr, void *__restrict__ tlist) {
     const PairDev &P = pairs[p];
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < P.nvirt; v += stride) {
-        long long rent, cent;
-        int layer, nl;
-        if (!vcell(S, P, v, rent, cent, layer, nl)) continue;
-        const int ra = P.rarity, nfr = P.tr / ra;
-        for (int i = 0; i < P.tr; ++i) {
-            const int k = nfr == 1 ? 0 : (i >= ra);
-            const int r = row_of(S, P, rent, k, i - k * ra, layer, nl);
-            if (r < 0) continue;
-            if (r >= S.nrows) {
-                atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
-                continue;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int ra = P.rarity, tr = P.tr;
+    const long long nvirt = P.nvirt, stride = (long long)gridDim.x * blockDim.x;
+    for (long long v0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); v0 < nvirt;
+         v0 += stride) {   // v0 is the same for a warp's lanes
+        const long long v = v0 + lane;
+        long long rent = 0, cent = 0;
+        int layer = 0, nl = 1;
+        const bool ok = v < nvirt && vcell(S, P, v, rent, cent, layer, nl);
+        for (int i0 = 0; i0 < tr; i0 += 4) {
+            int r[4], head[4], n[4];
+            long long at[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = i0 + q, k = i >= ra;
+                r[q] = ok && i < tr ? row_of(S, P, rent, k, i - k * ra, layer, nl) : -1;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (r[q] >= S.nrows) {
+                    atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
+                    r[q] = -1;
+                }
+                const int up = __shfl_up_sync(full, r[q], 1);
+                const unsigned heads = __ballot_sync(full, lane == 0 || up != r[q]);
+                head[q] = 31 - __clz(heads & (0xffffffffu >> (31 - lane)));
+                const unsigned later = heads & ~(0xffffffffu >> (31 - lane));
+                n[q] = (later ? __ffs(later) - 1 : 32) - lane;   // the run's length, at its head
             }
             if (pass == 0) {
-                atomicAdd((unsigned long long *)&cnt[r], 1ull);
-                if (!single_pair) atomicAdd(&cand[r], P.tc);
-            } else {
-                const long long pos = cnt[r] + atomicAdd(&fillpos[r], 1);
-                if (narrow)
-                    ((int *)tlist)[pos] = (int)v;
-                else
-                    tlist[pos] = ((long long)p << 56) | v;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (r[q] >= 0 && head[q] == lane) {
+                        atomicAdd(&cnt[r[q]], n[q]);
+                        if (cand) atomicAdd(&cand[r[q]], P.tc * n[q]);
+                    }
+                continue;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                at[q] = 0;
+                if (r[q] >= 0 && head[q] == lane)
+                    at[q] = ptr[r[q]] + atomicSub(&cnt[r[q]], n[q]) - n[q];
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const long long pos = __shfl_sync(full, at[q], head[q]) + (lane - head[q]);
+                if (r[q] < 0) continue;
+                if (EMODE == E_FLAT) ((int *)tlist)[pos] = (int)v;
+                else if (EMODE == E_LAYER) ((long long *)tlist)[pos] = rent << 32 | layer;
+                else ((long long *)tlist)[pos] = ((long long)p << 56) | v;
             }
         }
     }
+}
+
+// Column j of list entry pos: negative when there is none (a negative map
+// value, or one outside the column set, which is reported).
+template <int EMODE>
+__device__ __forceinline__ int entry_col(const SpDev &S, const PairDev *__restrict__ pairs,
+                                         const void *__restrict__ tlist, long long pos, int j) {
+    int c;
+    if (EMODE == E_FLAT) {
+        const PairDev &P = pairs[0];
+        c = __ldg(P.cmap + (long long)__ldg((const int *)tlist + pos) * P.carity + j);
+    } else if (EMODE == E_LAYER) {
+        const PairDev &P = pairs[0];
+        const long long w = __ldg((const long long *)tlist + pos);
+        const int ca = P.carity, k = j >= ca;
+        c = col_of(S, P, w >> 32, k, j - k * ca, (int)w, S.layers[1] - 1 - S.layers[0]);
+    } else {
+        const long long code = __ldg((const long long *)tlist + pos);
+        const PairDev &P = pairs[(int)(code >> 56)];
+        long long rent, cent;
+        int layer, nl;
+        if (!vcell(S, P, code & ((1ll << 56) - 1), rent, cent, layer, nl)) return -1;
+        const int ca = P.carity, k = j >= ca;
+        c = col_of(S, P, cent, k, j - k * ca, layer, nl);
+    }
+    if (c >= S.ncols) {
+        atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
+        c = -1;
+    }
+    return c;
+}
+
+// ---- rows of at most 256 candidate columns, all pairs with the same tc
+//
+// One warp takes a batch of rb consecutive rows; per row its lanes hold the
+// candidates in registers, CPL each (candidate i = column i % tc of the row's
+// i / tc-th list entry, so consecutive lanes read consecutive map values), and
+// find the distinct ones without atomics and without ever clearing a table:
+// every candidate writes its number into slot hash(column), the one that
+// reads its own number back owns the slot and writes its column there, and
+// the others compare: equal means a duplicate of the owner, unequal a
+// collision that another round with another hash settles (every round settles
+// at least one column per contended slot).  The owners' columns are packed
+// into a list by ballots and ordered by counting the smaller ones.
+//
+// The kernel is issue-bound (integer work on L2-resident maps): on the
+// 12.58 M-cell tet mesh the form it replaced (a warp per row too, columns
+// inserted one by one with shared-memory compare-and-swap after a
+// __match_any_sync) issued 489 warp instructions per row, this one 306.
+// A batch's columns are stored back to back at its first candidate's place,
+// so that the copy to the CSR array reads whole sectors.
+constexpr int ROW_CAP = 256, ROW_TS = 512, ROW_WARPS = 4, ROW_MINB = 10;
+
+// What a lane needs to fetch its candidates: fixed for a launch (the single
+// pair's arrays; tc and magic = 65536 / tc + 1, which divides exactly below
+// 256 candidates).
+struct RowArgs {
+    const int *cmap;
+    int ca, tc;
+    int vec4;     // rows of cmap are 16-byte aligned
+    unsigned magic;
+    int extra;   // a row's diagonal is a candidate of its own: 0 never, 1 only
+                 // of rows without entries (their own column is among the
+                 // entries' otherwise: one map on both sides), 2 always
+};
+
+template <int EMODE>
+__device__ __forceinline__ int small_col(const SpDev &S, const PairDev *__restrict__ pairs,
+                                         const RowArgs &A, const void *__restrict__ list, int e,
+                                         int j) {
+    if (EMODE != E_FLAT) return entry_col<EMODE>(S, pairs, list, e, j);
+    const int c = __ldg(A.cmap + ((long long)__ldg((const int *)list + e) * A.ca + j));
+    if (c >= S.ncols) {
+        atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
+        return -1;
+    }
+    return c;
+}
+
+template <int CPL, int EMODE>
+__device__ __forceinline__ int row_distinct(const SpDev &S, const PairDev *__restrict__ pairs,
+                                            const RowArgs &A, const void *__restrict__ list,
+                                            int ncand, int total, int diag_col,
+                                            unsigned short *ids, int *vals, int *uniq) {
+    constexpr int SH = 23;   // 32 - log2(ROW_TS)
+    static_assert(ROW_TS == 1 << (32 - SH), "table size and shift");
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int c[CPL];
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        const int i = lane + 32 * k;
+        const int e = (int)(((unsigned)i * A.magic) >> 16);   // i / tc
+        c[k] = -1;
+        if (i < ncand) c[k] = small_col<EMODE>(S, pairs, A, list, e, i - e * A.tc);
+        else if (i < total) c[k] = diag_col;
+    }
+    // First round, every lane alike (lanes without a candidate contend with
+    // the column -1, which is dropped when the owners are collected).
+    bool own[CPL], left[CPL], any = false;
+#pragma unroll
+    for (int k = 0; k < CPL; ++k)
+        ids[((unsigned)c[k] * 2654435761u) >> SH] = (unsigned short)(lane + 32 * k);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        const unsigned h = ((unsigned)c[k] * 2654435761u) >> SH;
+        own[k] = ids[h] == lane + 32 * k;
+        if (own[k]) vals[h] = c[k];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        left[k] = vals[((unsigned)c[k] * 2654435761u) >> SH] != c[k];
+        any |= left[k];
+    }
+    unsigned mult = 2654435761u;
+    while (__any_sync(full, any)) {
+        __syncwarp();
+        mult *= 0x9E3779B1u;   // another odd multiplier
+#pragma unroll
+        for (int k = 0; k < CPL; ++k)
+            if (left[k]) ids[((unsigned)c[k] * mult) >> SH] = (unsigned short)(lane + 32 * k);
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < CPL; ++k)
+            if (left[k] && ids[((unsigned)c[k] * mult) >> SH] == lane + 32 * k) {
+                own[k] = true;
+                vals[((unsigned)c[k] * mult) >> SH] = c[k];
+            }
+        __syncwarp();
+        any = false;
+#pragma unroll
+        for (int k = 0; k < CPL; ++k) {
+            left[k] = left[k] && vals[((unsigned)c[k] * mult) >> SH] != c[k];
+            any |= left[k];
+        }
+    }
+    int u = 0;
+#pragma unroll
+    for (int k = 0; k < CPL; ++k) {
+        const bool mine = own[k] && c[k] >= 0;
+        const unsigned b = __ballot_sync(full, mine);
+        if (mine) uniq[u + __popc(b & ((1u << lane) - 1))] = c[k];
+        u += __popc(b);
+    }
+    return u;
+}
+
+// Ascending order of the u distinct columns in uniq (room for a power of two,
+// 16-byte aligned) into out.
+__device__ __forceinline__ void row_sorted(int *uniq, int u, int *__restrict__ out) {
+    const int lane = threadIdx.x & 31;
+    if (u <= 16) {
+        // each half of the warp counts among eight of sixteen places
+        if (lane < 16) uniq[u + lane] = INT_MAX;
+        __syncwarp();
+        const int x = uniq[lane & 15], half = lane >> 4 << 3;
+        const int4 v = *(const int4 *)(uniq + half), w = *(const int4 *)(uniq + half + 4);
+        int rank = (v.x < x) + (v.y < x) + (v.z < x) + (v.w < x) + (w.x < x) + (w.y < x) +
+                   (w.z < x) + (w.w < x);
+        rank += __shfl_xor_sync(0xffffffffu, rank, 16);
+        if (lane < u) out[rank] = x;
+        return;
+    }
+    if (u <= 32) {
+        if (lane < 4) uniq[u + lane] = INT_MAX;
+        __syncwarp();
+        const int x = lane < u ? uniq[lane] : INT_MAX;
+        int rank = 0;
+        for (int j = 0; j < u; j += 4) {
+            const int4 v = *(const int4 *)(uniq + j);
+            rank += (v.x < x) + (v.y < x) + (v.z < x) + (v.w < x);
+        }
+        if (lane < u) out[rank] = x;
+        return;
+    }
+    int P2 = 64;
+    while (P2 < u) P2 <<= 1;
+    for (int i = u + lane; i < P2; i += 32) uniq[i] = INT_MAX;
+    __syncwarp();
+    for (int k = 2; k <= P2; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = lane; i < P2; i += 32) {
+                const int ixj = i ^ j;
+                if (ixj > i) {
+                    const int a = uniq[i], b = uniq[ixj];
+                    if ((a > b) == ((i & k) == 0)) {
+                        uniq[i] = b;
+                        uniq[ixj] = a;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    for (int i = lane; i < u; i += 32) out[i] = uniq[i];
+}
+
+// Ascending order of v[0..N), N a power of two: a bitonic network written as a
+// recursion, so that every index is a constant and v stays in registers.
+template <int N, int K = 2, int J = 1>
+__device__ __forceinline__ void sort_network(unsigned (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+        if ((i ^ J) > i) {
+            const unsigned a = v[i], b = v[i ^ J], lo = a < b ? a : b, hi = a < b ? b : a;
+            v[i] = i & K ? hi : lo;
+            v[i ^ J] = i & K ? lo : hi;
+        }
+    if constexpr (J > 1) sort_network<N, K, J / 2>(v);
+    else if constexpr (K < N) sort_network<N, 2 * K, K>(v);
+}
+
+// The other way to find a batch's distinct columns: one lane per row.  A lane
+// enters its row's candidates one by one into an open-addressing table of its
+// own (THREAD_TS places in shared memory; lane l's places all lie in bank l,
+// so no two lanes conflict), sorts the distinct ones in registers, and the
+// warp stores the rows packed.  There are no ballots, barriers or shuffles per
+// row: 197 warp instructions per row of the tet mesh against 306 for the
+// warp-per-row form, 0.29 against 0.39 ms at 6 M cells (bound by issue slots
+// and the latency of the lists and map rows; tables of 40-64 places take fewer
+// probes but leave fewer warps resident: 0.28-0.35 ms; entering four columns
+// together, a probe of each lane at a time, 0.34 ms).  A batch with a row of
+// more than THREAD_MAX distinct columns returns -1 and runs the other form.
+// Returns the columns stored; *u_out = this lane's.
+constexpr int THREAD_TS = 32, THREAD_MAX = 28;
+
+template <int EMODE>
+__device__ __forceinline__ int rows_by_lane(const SpDev &S, const PairDev *__restrict__ pairs,
+                                            const RowArgs &A, const void *__restrict__ tlist,
+                                            long long e0, int m, bool diag, int r, int *T, int *out,
+                                            int *u_out) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const void *list = (const char *)tlist + e0 * (EMODE == E_FLAT ? 4 : 8);
+#pragma unroll
+    for (int s = 0; s < THREAD_TS; ++s) T[s * 32 + lane] = -1;
+    const int nl = EMODE == E_LAYER ? S.layers[1] - 1 - S.layers[0] : 1;   // cell layers
+    int u = 0;
+    bool over = false;
+    auto place = [&](int c) { return ((unsigned)c * 2654435761u) >> 27; };   // 32 - log2(THREAD_TS)
+    // a row's own column is entered at once, and met again in every entry when
+    // the pair is one map on both sides
+    const int own = A.extra == 1 && m && r < S.ncols ? r : -1;
+    if (diag || own >= 0) {
+        T[place(r) * 32 + lane] = r;
+        u = 1;
+    }
+    // Enter up to four columns (negative: none).
+    auto enter = [&](int (&c)[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (c[k] >= S.ncols) {
+                atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
+                c[k] = -1;
+            }
+            if (c[k] < 0 || c[k] == own || over) continue;
+            unsigned h = place(c[k]);
+            for (;;) {
+                const int v = T[h * 32 + lane];
+                if (v == c[k]) break;
+                if (v < 0) {
+                    if (u < THREAD_MAX) T[h * 32 + lane] = c[k];
+                    else over = true;
+                    ++u;
+                    break;
+                }
+                h = (h + 1) & (THREAD_TS - 1);   // a free place is left, so this ends
+            }
+        }
+    };
+    for (int e = 0; e < m && !over; ++e) {
+        const int *row = nullptr, *coff = nullptr, *cq = nullptr;
+        int layer = 0;
+        if (EMODE == E_FLAT) {
+            row = A.cmap + (long long)__ldg((const int *)list + e) * A.ca;
+        } else if (EMODE == E_LAYER) {
+            const long long w = __ldg((const long long *)list + e);
+            row = A.cmap + (w >> 32) * A.ca;
+            layer = (int)w;
+            coff = pairs[0].coff;
+            cq = pairs[0].cq;
+        }
+        for (int j0 = 0; j0 < A.tc && !over; j0 += 4) {
+            int c[4];
+            if (EMODE == E_FLAT && A.vec4) {
+                const int4 v = __ldg((const int4 *)(row + j0));
+                c[0] = v.x;
+                c[1] = v.y;
+                c[2] = v.z;
+                c[3] = v.w;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int j = j0 + q, k = j >= A.ca, jr = j - k * A.ca;
+                    c[q] = -1;
+                    if (j >= A.tc) continue;
+                    if (EMODE == E_CODE) c[q] = entry_col<EMODE>(S, pairs, list, e, j);
+                    else if (EMODE == E_FLAT) c[q] = __ldg(row + j);
+                    else c[q] = __ldg(row + jr) + __ldg(coff + jr) * ext_term(layer, k, __ldg(cq + jr), nl);
+                }
+            }
+            enter(c);
+        }
+    }
+    if (__any_sync(full, over)) return -1;
+    int before = u;   // inclusive sum over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(full, before, o);
+        if (lane >= o) before += y;
+    }
+    const int total = __shfl_sync(full, before, 31);
+    before -= u;
+    if (__reduce_max_sync(full, (unsigned)u) <= 16) {
+        // the free places go (in place: the k-th value lies at or after k)
+        int k = 0;
+#pragma unroll
+        for (int s = 0; s < THREAD_TS; ++s) {
+            const int v = T[s * 32 + lane];
+            if (v >= 0) T[k++ * 32 + lane] = v;
+        }
+        unsigned v[16];
+#pragma unroll
+        for (int s = 0; s < 16; ++s) v[s] = s < u ? (unsigned)T[s * 32 + lane] : 0xffffffffu;
+        sort_network(v);
+        __syncwarp();
+#pragma unroll
+        for (int s = 0; s < 16; ++s)
+            if (s < u) T[before + s] = (int)v[s];
+    } else {
+        unsigned v[THREAD_TS];   // a free place, -1, is the largest unsigned value
+#pragma unroll
+        for (int s = 0; s < THREAD_TS; ++s) v[s] = (unsigned)T[s * 32 + lane];
+        sort_network(v);
+        __syncwarp();
+#pragma unroll
+        for (int s = 0; s < THREAD_MAX; ++s)
+            if (s < u) T[before + s] = (int)v[s];
+    }
+    __syncwarp();
+    for (int i = lane; i < total; i += 32) out[i] = T[i];
+    *u_out = u;
+    return total;
+}
+
+// First candidate place of row r (one more per row for the diagonal).
+__device__ __forceinline__ long long batch_base(const long long *__restrict__ ptr, long long r,
+                                                int tc, int diag) {
+    return ptr[r] * tc + (diag ? r : 0);
+}
+
+template <int EMODE>
+__global__ void __launch_bounds__(32 * ROW_WARPS, ROW_MINB)
+    k_rows_small(SpDev S, const PairDev *__restrict__ pairs, RowArgs A,
+                 const long long *__restrict__ ptr, const void *__restrict__ tlist, int rb,
+                 int *__restrict__ tmp, int *__restrict__ rowcount, int *__restrict__ big) {
+    // per warp: the lanes' tables, or the places' columns, the packed columns
+    // and the places' candidate numbers
+    constexpr int WORDS = ROW_TS + ROW_CAP + 16 + ROW_TS / 2;
+    static_assert(WORDS >= 32 * THREAD_TS, "shared memory of a warp");
+    __shared__ __align__(16) int smem[ROW_WARPS][WORDS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int *vals = smem[warp], *uniq = vals + ROW_TS;
+    unsigned short *ids = (unsigned short *)(uniq + ROW_CAP + 16);
+    const long long r0 = ((long long)blockIdx.x * ROW_WARPS + warp) * rb;
+    if (r0 >= S.nrows) return;
+    const int n = (int)(S.nrows - r0 < rb ? S.nrows - r0 : rb);
+    int entries = 0;   // of row r0 + lane, cut off just above the limit
+    long long e0 = 0;
+    if (lane < n) {
+        e0 = ptr[r0 + lane];
+        const long long m = ptr[r0 + lane + 1] - e0;
+        entries = m > ROW_CAP ? ROW_CAP + 1 : (int)m;
+    }
+    int *out = tmp + batch_base(ptr, r0, A.tc, S.set_diag);
+    if (rb == 32) {
+        const bool diag = lane < n && A.extra && r0 + lane < S.ncols &&
+                          (A.extra == 2 || entries == 0);
+        int u = 0;
+        if (!__any_sync(0xffffffffu, entries * A.tc > ROW_CAP) &&
+            rows_by_lane<EMODE>(S, pairs, A, tlist, e0, entries, diag, (int)(r0 + lane), vals, out,
+                                &u) >= 0) {
+            if (lane < n) rowcount[r0 + lane] = u;
+            return;
+        }
+        __syncwarp();
+    }
+    const char *list = (const char *)tlist + ptr[r0] * (EMODE == E_FLAT ? 4 : 8);
+    int count = 0;
+    for (int i = 0; i < n; ++i) {
+        const int m = __shfl_sync(0xffffffffu, entries, i);
+        const int diag = A.extra && r0 + i < S.ncols && (A.extra == 2 || m == 0);
+        if (m > ROW_CAP || m * A.tc + diag > ROW_CAP) {   // the caller falls back to k_rows
+            if (lane == 0) atomicOr(big, 1);
+            return;
+        }
+        const int nc = m * A.tc, tot = nc + diag, dc = (int)(r0 + i);
+        int u = 0;
+        if (tot <= 32) u = row_distinct<1, EMODE>(S, pairs, A, list, nc, tot, dc, ids, vals, uniq);
+        else if (tot <= 64) u = row_distinct<2, EMODE>(S, pairs, A, list, nc, tot, dc, ids, vals, uniq);
+        else if (tot <= 96) u = row_distinct<3, EMODE>(S, pairs, A, list, nc, tot, dc, ids, vals, uniq);
+        else if (tot <= 128) u = row_distinct<4, EMODE>(S, pairs, A, list, nc, tot, dc, ids, vals, uniq);
+        else u = row_distinct<8, EMODE>(S, pairs, A, list, nc, tot, dc, ids, vals, uniq);
+        __syncwarp();
+        row_sorted(uniq, u, out);
+        __syncwarp();
+        if (lane == i) count = u;
+        out += u;
+        list += m * (EMODE == E_FLAT ? 4 : 8);
+    }
+    if (lane < n) rowcount[r0 + lane] = count;
+}
+
+// One warp per batch of k_rows_small: its columns, back to back in tmp, to
+// the CSR column array.
+__global__ void __launch_bounds__(256)
+    k_batches_copy(long long nrows, const long long *__restrict__ ptr, int tc, int diag, int rb,
+                   const int *__restrict__ tmp, const long long *__restrict__ rowptr,
+                   int *__restrict__ colidx) {
+    const int lane = threadIdx.x & 31;
+    const long long r0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * rb;
+    if (r0 >= nrows) return;
+    const long long r1 = r0 + rb < nrows ? r0 + rb : nrows;
+    const long long o = rowptr[r0];
+    const int n = (int)(rowptr[r1] - o);
+    const int *__restrict__ src = tmp + batch_base(ptr, r0, tc, diag);
+    int *__restrict__ dst = colidx + o;
+#pragma unroll 8
+    for (int i = lane; i < n; i += 32) dst[i] = __ldg(src + i);
 }
 
 // Candidate count of row i: cand[i], or its incidences times tc when tc > 0
@@ -190,18 +668,18 @@ __device__ __forceinline__ void row_insert(int c, int *tab, unsigned mask, int t
     atomicOr(err, OP2G_DEVERR_CAPACITY);  // table full: cannot happen (tsize >= 2 x candidates)
 }
 
-// SIMPLE: one (row map, column map) pair over a flat set with no composed
-// maps, so the transpose list holds 32-bit entity numbers and an entry's
-// candidate columns are one row of the column map.  The warp then walks the incident
-// cells in warp-uniform rounds and, per column slot, lets only the first of
-// the lanes holding the same column insert it (__match_any_sync): on a mesh
-// a vertex's own column recurs in every incident cell, and most neighbours
-// in several, so this removes about half of the shared-memory atomics.
-template <bool SIMPLE>
+// This is the form for rows of more than ROW_CAP candidates and for pairs
+// that bring different numbers of them.
+// For E_FLAT lists the warp walks the incident cells in warp-uniform rounds
+// and, per column slot, lets only the first of the lanes holding the same
+// column insert it (__match_any_sync): on a mesh a vertex's own column recurs
+// in every incident cell, and most neighbours in several, so this removes
+// about half of the shared-memory atomics.
+template <int EMODE>
 __global__ void k_rows(SpDev S, const PairDev *__restrict__ pairs,
-                       const long long *__restrict__ tptr, const long long *__restrict__ tlist,
+                       const long long *__restrict__ tptr, const void *__restrict__ tlist,
                        int tsize, int ucap, const long long *__restrict__ candptr,
-                       int *__restrict__ tmp, long long *__restrict__ rowcount) {
+                       int *__restrict__ tmp, int *__restrict__ rowcount) {
     extern __shared__ int smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int wpb = blockDim.x >> 5;
@@ -218,41 +696,26 @@ __global__ void k_rows(SpDev S, const PairDev *__restrict__ pairs,
         if (lane == 0) hdr[0] = 0;
         __syncwarp();
         const long long e0 = tptr[r], e1 = tptr[r + 1];
-        if (SIMPLE) {
-            const int *cmap = pairs[0].cmap;
+        if (EMODE == E_FLAT) {
             const int ca = pairs[0].carity;
             for (long long b = e0; b < e1; b += 32) {  // warp-uniform rounds
                 const long long e = b + lane;
-                const int *crow =
-                    e < e1 ? cmap + (long long)((const int *)tlist)[e] * ca : nullptr;
                 for (int j = 0; j < ca; ++j) {
-                    int c = crow ? __ldg(crow + j) : -1;
-                    if (c >= S.ncols) {
-                        atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
-                        c = -1;
-                    }
+                    const int c = e < e1 ? entry_col<EMODE>(S, pairs, tlist, e, j) : -1;
                     const unsigned same = __match_any_sync(0xffffffffu, c);
                     if (c >= 0 && (__ffs(same) - 1) == lane)
                         row_insert(c, tab, mask, tsize, uniq, uslot, hdr, S.err);
                 }
             }
-        }
-        for (long long e = e0 + lane; !SIMPLE && e < e1; e += 32) {
-            const long long code = tlist[e];
-            const PairDev &P = pairs[(int)(code >> 56)];
-            long long rent, cent;
-            int layer, nl;
-            if (!vcell(S, P, code & ((1ll << 56) - 1), rent, cent, layer, nl)) continue;
-            const int ca = P.carity, nfc = P.tc / ca;
-            for (int j = 0; j < P.tc; ++j) {
-                const int k = nfc == 1 ? 0 : (j >= ca);
-                const int c = col_of(S, P, cent, k, j - k * ca, layer, nl);
-                if (c < 0) continue;
-                if (c >= S.ncols) {
-                    atomicOr(S.err, OP2G_DEVERR_MAP_BOUNDS);
-                    continue;
+        } else {
+            for (long long e = e0 + lane; e < e1; e += 32) {
+                const int tc = EMODE == E_LAYER
+                                   ? pairs[0].tc
+                                   : pairs[(int)(((const long long *)tlist)[e] >> 56)].tc;
+                for (int j = 0; j < tc; ++j) {
+                    const int c = entry_col<EMODE>(S, pairs, tlist, e, j);
+                    if (c >= 0) row_insert(c, tab, mask, tsize, uniq, uslot, hdr, S.err);
                 }
-                row_insert(c, tab, mask, tsize, uniq, uslot, hdr, S.err);
             }
         }
         if (S.set_diag && r < S.ncols && lane == 0)
@@ -323,14 +786,16 @@ namespace op2g {
 // (shared with the staging plan in op2g_stage.cu)
 constexpr int SCAN_T = 1024, SCAN_V = 4, SCAN_B = SCAN_T * SCAN_V;
 
-__global__ void __launch_bounds__(SCAN_T) k_scan_block(long long *__restrict__ d, long long n,
+// src: what is summed (d itself, or 32-bit counts)
+template <class T>
+__global__ void __launch_bounds__(SCAN_T) k_scan_block(const T *src, long long *d, long long n,
                                                        long long *__restrict__ sums) {
     __shared__ long long ws[32];
     const long long b0 = (long long)blockIdx.x * SCAN_B + (long long)threadIdx.x * SCAN_V;
     long long v[SCAN_V], t = 0;
 #pragma unroll
     for (int k = 0; k < SCAN_V; ++k) {
-        v[k] = (b0 + k < n) ? d[b0 + k] : 0;
+        v[k] = (b0 + k < n) ? (long long)src[b0 + k] : 0;
         t += v[k];
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -373,22 +838,28 @@ size_t scan_tmp_elems(long long n) {
     return tot + 1;
 }
 
-// Exclusive in-place scan of d[0..n); tmp needs scan_tmp_elems(n) elements.
-op2g_status scan_exclusive(long long *d, long long n, long long *tmp, cudaStream_t st) {
+// Exclusive scan of src[0..n) into d (which may be src); tmp needs
+// scan_tmp_elems(n) elements.
+template <class T>
+op2g_status scan_from(const T *src, long long *d, long long n, long long *tmp, cudaStream_t st) {
     if (n <= 0) return OP2G_OK;
     if (n <= SCAN_B) {
-        k_scan_block<<<1, SCAN_T, 0, st>>>(d, n, nullptr);
+        k_scan_block<<<1, SCAN_T, 0, st>>>(src, d, n, (long long *)nullptr);
         CK(cudaGetLastError());
         return OP2G_OK;
     }
     const long long nb = (n + SCAN_B - 1) / SCAN_B;
-    k_scan_block<<<(unsigned)nb, SCAN_T, 0, st>>>(d, n, tmp);
+    k_scan_block<<<(unsigned)nb, SCAN_T, 0, st>>>(src, d, n, tmp);
     CK(cudaGetLastError());
-    op2g_status s = scan_exclusive(tmp, nb, tmp + nb, st);
+    op2g_status s = scan_from(tmp, tmp, nb, tmp + nb, st);
     if (s != OP2G_OK) return s;
     k_scan_add<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d, n, tmp);
     CK(cudaGetLastError());
     return OP2G_OK;
+}
+
+op2g_status scan_exclusive(long long *d, long long n, long long *tmp, cudaStream_t st) {
+    return scan_from(d, d, n, tmp, st);
 }
 
 }  // namespace op2g
@@ -396,13 +867,16 @@ op2g_status scan_exclusive(long long *d, long long n, long long *tmp, cudaStream
 namespace {
 
 using op2g::scan_exclusive;
+using op2g::scan_from;
 using op2g::scan_tmp_elems;
 
 // ------------------------------------------------------- sparsity driver
 struct SpLayout {
-    size_t off_cnt, off_cand, off_fill, off_tlist, off_scan, off_pairs, off_misc, off_candptr,
+    size_t off_cnt, off_ptr, off_cand, off_tlist, off_scan, off_pairs, off_misc, off_candptr,
         off_tmp, total;
     long long ninc, ncand;
+    int emode;   // what the transpose list holds
+    int tc;      // candidate columns per list entry, 0 when the pairs differ
 };
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -471,12 +945,21 @@ op2g_status sp_prepare(const op2g_sparsity_desc *d, std::vector<PairDev> &pairs,
         L.ncand += P.nvirt * P.tr * P.tc;
     }
     L.ncand += d->nrows;  // diagonal entries
+    L.emode = E_CODE;
+    L.tc = d->npairs ? pairs[0].tc : 0;
+    for (const PairDev &P : pairs)
+        if (P.tc != L.tc) L.tc = 0;
+    if (d->npairs == 1 && !pairs[0].nrc && !pairs[0].ncc) {
+        if (!d->extruded) L.emode = E_FLAT;   // set sizes are int32
+        else if (d->constant_layers) L.emode = E_LAYER;
+    }
     const long long n1 = d->nrows + 1;
     size_t off = 0;
-    L.off_cnt = off; off = align256(off + sizeof(long long) * n1);
-    L.off_cand = off; off = align256(off + sizeof(int) * (d->nrows + 1));
-    L.off_fill = off; off = align256(off + sizeof(int) * (d->nrows + 1));
-    L.off_tlist = off; off = align256(off + sizeof(long long) * (L.ninc > 0 ? L.ninc : 1));
+    L.off_cnt = off; off = align256(off + sizeof(int) * n1);
+    L.off_ptr = off; off = align256(off + sizeof(long long) * n1);
+    L.off_cand = off; off = align256(off + sizeof(int) * (L.tc ? 1 : n1));
+    L.off_tlist = off; off = align256(off + (L.emode == E_FLAT ? sizeof(int) : sizeof(long long)) *
+                                                (L.ninc > 0 ? L.ninc : 1));
     L.off_scan = off; off = align256(off + sizeof(long long) * scan_tmp_elems(n1));
     L.off_pairs = off; off = align256(off + sizeof(PairDev) * (d->npairs ? d->npairs : 1));
     L.off_misc = off; off = align256(off + 64);
@@ -493,11 +976,10 @@ int sms_of_current() {
     return n > 0 ? n : 1;
 }
 
-op2g_status sp_rows_launch(const SpDev &S, const PairDev *pd, bool simple,
-                           const long long *tptr, const long long *tlist, int max_cand,
-                           const long long *candptr, int *tmp, long long *rowcount,
-                           cudaStream_t st) {
-    if (S.nrows == 0) return OP2G_OK;
+template <int EMODE>
+op2g_status sp_rows_launch(const SpDev &S, const PairDev *pd, const long long *tptr,
+                           const void *tlist, int max_cand, const long long *candptr, int *tmp,
+                           int *rowcount, cudaStream_t st) {
     int tsize = 32;
     while (tsize < 2 * max_cand) tsize <<= 1;
     int ucap = 32;
@@ -509,21 +991,14 @@ op2g_status sp_rows_launch(const SpDev &S, const PairDev *pd, bool simple,
     const size_t smem = per * wpb;
     if (smem > 227 * 1024)
         return op2g::fail(OP2G_ERR_CAPACITY, "a sparsity row has more than 18,000 candidate columns");
-    if (smem > 48 * 1024) {
-        CK(cudaFuncSetAttribute(k_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (smem > 48 * 1024)
+        CK(cudaFuncSetAttribute(k_rows<EMODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)smem));
-        CK(cudaFuncSetAttribute(k_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
-    }
     long long blocks = (S.nrows + wpb - 1) / wpb;
     const long long capb = (long long)sms_of_current() * 32;
     if (blocks > capb) blocks = capb;
-    if (simple)
-        k_rows<true><<<(unsigned)blocks, 32 * wpb, smem, st>>>(S, pd, tptr, tlist, tsize, ucap,
-                                                               candptr, tmp, rowcount);
-    else
-        k_rows<false><<<(unsigned)blocks, 32 * wpb, smem, st>>>(S, pd, tptr, tlist, tsize, ucap,
-                                                                candptr, tmp, rowcount);
+    k_rows<EMODE><<<(unsigned)blocks, 32 * wpb, smem, st>>>(S, pd, tptr, tlist, tsize, ucap,
+                                                            candptr, tmp, rowcount);
     CK(cudaGetLastError());
     return OP2G_OK;
 }
@@ -535,12 +1010,106 @@ unsigned grid_for_rows(long long nrows) {
     return (unsigned)(g < 1 ? 1 : g);
 }
 
-// State kept in the workspace between count and fill (the candidate capacity).
+// State kept in the workspace between count and fill.
 struct SpMisc {
     int max_cand;
     int err;
-    int cap;
+    int big;          // a row has more than ROW_CAP candidates
+    int small;        // the pattern came from k_rows_small (batches of rb rows)
+    int done;         // op2g_sparsity_count succeeded
+    long long total;
 };
+
+// Rows per warp of k_rows_small: 32, one per lane, where that gives every SM
+// RB_WARPS warps; on smaller meshes fewer, for more warps (16 at most: 32
+// stands for the lane-per-row form).  Measured, whole pattern builds, lane per
+// row against warp per row: 68,921 rows of P1 tets 164 against 154 us, 135,168
+// rows of prisms 166 against 203 us.
+constexpr int RB_WARPS = 20;
+int rows_per_batch(long long nrows) {
+    const long long sms = sms_of_current();
+    if (nrows >= sms * RB_WARPS * 32) return 32;
+    const long long rb = nrows / (sms * 64);
+    return rb < 1 ? 1 : rb > 16 ? 16 : (int)rb;
+}
+
+// Row counts (int, into cnt) and columns (into tmp) of every row, from the
+// transpose list; *small tells which of the two forms ran.
+template <int EMODE>
+op2g_status sp_rows(const op2g_sparsity_desc *d, const std::vector<PairDev> &pairs, const SpDev &S,
+                    const SpLayout &L, char *w, int rb, cudaStream_t st) {
+    int *cnt = (int *)(w + L.off_cnt), *cand = L.tc ? nullptr : (int *)(w + L.off_cand);
+    long long *ptr = (long long *)(w + L.off_ptr);
+    void *tlist = w + L.off_tlist;
+    const PairDev *pd = (const PairDev *)(w + L.off_pairs);
+    SpMisc *misc = (SpMisc *)(w + L.off_misc);
+    long long *scan = (long long *)(w + L.off_scan);
+    int *tmp = (int *)(w + L.off_tmp);
+    const long long n1 = d->nrows + 1, capb = (long long)sms_of_current() * 16;
+    if (rb > 0) {   // list, then rows in batches of rb
+        for (int pass = 0; pass < 2; ++pass) {
+            for (size_t p = 0; p < pairs.size(); ++p) {
+                long long nb = (pairs[p].nvirt + 255) / 256;
+                if (nb == 0) continue;
+                if (nb > capb) nb = capb;
+                k_incidence<EMODE><<<(unsigned)nb, 256, 0, st>>>(S, pd, (int)p, pass, cnt, cand,
+                                                                 ptr, tlist);
+                CK(cudaGetLastError());
+            }
+            if (pass == 0) {
+                op2g_status s = scan_from(cnt, ptr, n1, scan, st);
+                if (s != OP2G_OK) return s;
+            }
+        }
+        if (L.tc && d->nrows > 0) {
+            const long long nb = (d->nrows + (long long)rb * ROW_WARPS - 1) / ((long long)rb * ROW_WARPS);
+            const PairDev &P = pairs[0];
+            RowArgs A;
+            A.cmap = P.cmap;
+            A.ca = P.carity;
+            A.tc = L.tc;
+            A.vec4 = P.carity % 4 == 0 && (uintptr_t)P.cmap % 16 == 0;
+            A.magic = 65536u / (unsigned)L.tc + 1u;
+            // one map on both sides: an entry of row r has column r (an
+            // extruded map's layer terms are then the same ones too)
+            const bool same = pairs.size() == 1 && P.rmap == P.cmap && P.rarity == P.carity &&
+                              !P.nrc && !P.ncc &&
+                              !memcmp(P.roff, P.coff, sizeof P.roff) &&
+                              !memcmp(P.rq, P.cq, sizeof P.rq);
+            A.extra = !d->set_diag ? 0 : same ? 1 : 2;
+            k_rows_small<EMODE><<<(unsigned)nb, 32 * ROW_WARPS, 0, st>>>(S, pd, A, ptr, tlist, rb,
+                                                                         tmp, cnt, &misc->big);
+            CK(cudaGetLastError());
+        }
+        return OP2G_OK;
+    }
+    // rows of any size, at their candidate offsets
+    if (d->nrows == 0) return OP2G_OK;
+    long long nb = (d->nrows + 255) / 256;
+    if (nb > capb) nb = capb;
+    const int diag = d->set_diag ? 1 : 0;
+    k_max_cand<<<(unsigned)nb, 256, 0, st>>>(cand, ptr, L.tc, d->nrows, diag, &misc->max_cand);
+    CK(cudaGetLastError());
+    long long *candptr = (long long *)(w + L.off_candptr);
+    k_cand_sizes<<<(unsigned)nb, 256, 0, st>>>(cand, ptr, L.tc, d->nrows, d->ncols, diag, candptr);
+    CK(cudaGetLastError());
+    CK(cudaMemsetAsync(candptr + d->nrows, 0, sizeof(long long), st));
+    op2g_status s = scan_exclusive(candptr, n1, scan, st);
+    if (s != OP2G_OK) return s;
+    int max_cand = 0;
+    CK(cudaMemcpyAsync(&max_cand, &misc->max_cand, sizeof max_cand, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    return sp_rows_launch<EMODE>(S, pd, ptr, tlist, max_cand > 1 ? max_cand : 1, candptr, tmp, cnt, st);
+}
+
+op2g_status sp_rows_any(const op2g_sparsity_desc *d, const std::vector<PairDev> &pairs,
+                        const SpDev &S, const SpLayout &L, char *w, int rb, cudaStream_t st) {
+    switch (L.emode) {
+        case E_FLAT: return sp_rows<E_FLAT>(d, pairs, S, L, w, rb, st);
+        case E_LAYER: return sp_rows<E_LAYER>(d, pairs, S, L, w, rb, st);
+        default: return sp_rows<E_CODE>(d, pairs, S, L, w, rb, st);
+    }
+}
 
 }  // namespace
 
@@ -567,85 +1136,55 @@ op2g_status op2g_sparsity_count(const op2g_sparsity_desc *d, void *ws, size_t ws
     if (!rowptr) return op2g::fail(OP2G_ERR_INVALID, "rowptr is NULL");
     cudaStream_t st = (cudaStream_t)stream;
     char *w = (char *)ws;
-    long long *cnt = (long long *)(w + L.off_cnt);
-    int *cand = (int *)(w + L.off_cand);
-    int *fill = (int *)(w + L.off_fill);
-    long long *tlist = (long long *)(w + L.off_tlist);
-    long long *scan = (long long *)(w + L.off_scan);
-    PairDev *pd = (PairDev *)(w + L.off_pairs);
     SpMisc *misc = (SpMisc *)(w + L.off_misc);
+    long long *scan = (long long *)(w + L.off_scan);
+    int *cnt = (int *)(w + L.off_cnt);
     S.err = &misc->err;
     const long long n1 = d->nrows + 1;
-    CK(cudaMemsetAsync(cnt, 0, sizeof(long long) * n1, st));
-    CK(cudaMemsetAsync(cand, 0, sizeof(int) * n1, st));
-    CK(cudaMemsetAsync(fill, 0, sizeof(int) * n1, st));
+    CK(cudaMemsetAsync(cnt, 0, sizeof(int) * n1, st));
+    if (!L.tc) CK(cudaMemsetAsync(w + L.off_cand, 0, sizeof(int) * n1, st));
     CK(cudaMemsetAsync(misc, 0, sizeof(SpMisc), st));
     if (!pairs.empty())
-        CK(cudaMemcpyAsync(pd, pairs.data(), sizeof(PairDev) * pairs.size(), cudaMemcpyHostToDevice, st));
-    const long long capb = (long long)sms_of_current() * 16;
-    const int single = pairs.size() == 1 ? 1 : 0;
-    const int tc1 = single ? pairs[0].tc : 0;  // candidates per incidence with one pair
-    // one pair over a flat set without composed maps: the transpose list
-    // holds entity numbers (32-bit: set sizes are int32)
-    const bool simple = single && !d->extruded && pairs[0].nrc == 0 && pairs[0].ncc == 0;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (size_t p = 0; p < pairs.size(); ++p) {
-            long long nb = (pairs[p].nvirt + 255) / 256;
-            if (nb == 0) continue;
-            if (nb > capb) nb = capb;
-            k_incidence<<<(unsigned)nb, 256, 0, st>>>(S, pd, (int)p, pass, single,
-                                                      simple ? 1 : 0, cnt, cand, fill, tlist);
-            CK(cudaGetLastError());
-        }
-        if (pass == 0) {
-            s = scan_exclusive(cnt, n1, scan, st);
+        CK(cudaMemcpyAsync(w + L.off_pairs, pairs.data(), sizeof(PairDev) * pairs.size(),
+                           cudaMemcpyHostToDevice, st));
+    const int rb = rows_per_batch(d->nrows);
+    s = sp_rows_any(d, pairs, S, L, w, rb, st);
+    if (s != OP2G_OK) return s;
+    SpMisc hm;
+    memset(&hm, 0, sizeof hm);
+    hm.small = L.tc != 0;
+    for (;;) {
+        // Row pointers and one read-back of the total and the flags.  Without
+        // a common tc, or when a row had more than ROW_CAP candidates, the
+        // rows are made (again) by the form without that limit.
+        const int small = hm.small;
+        if (!small) {
+            int err = 0;
+            CK(cudaMemcpyAsync(&err, &misc->err, sizeof err, cudaMemcpyDeviceToHost, st));
+            CK(cudaStreamSynchronize(st));
+            if (err & OP2G_DEVERR_MAP_BOUNDS)
+                return op2g::fail(OP2G_ERR_BOUNDS, "a map value is outside the row or column set");
+            s = sp_rows_any(d, pairs, S, L, w, 0, st);
             if (s != OP2G_OK) return s;
         }
+        s = scan_from(cnt, (long long *)rowptr, n1, scan, st);
+        if (s != OP2G_OK) return s;
+        CK(cudaMemcpyAsync(&misc->total, rowptr + d->nrows, sizeof(long long),
+                           cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(&hm, misc, sizeof hm, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        hm.small = small;
+        if (!(small && hm.big)) break;
+        hm.small = 0;
     }
-    if (d->nrows > 0) {
-        long long nb = (d->nrows + 255) / 256;
-        if (nb > capb) nb = capb;
-        k_max_cand<<<(unsigned)nb, 256, 0, st>>>(cand, cnt, tc1, d->nrows, d->set_diag ? 1 : 0,
-                                                 &misc->max_cand);
-        CK(cudaGetLastError());
-    }
-    SpMisc hm;
-    CK(cudaMemcpyAsync(&hm, misc, sizeof hm, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
     if (hm.err & OP2G_DEVERR_MAP_BOUNDS)
         return op2g::fail(OP2G_ERR_BOUNDS, "a map value is outside the row or column set");
-    // candidate offsets (upper bound of each row's distinct columns)
-    long long *candptr = (long long *)(w + L.off_candptr);
-    int *tmp = (int *)(w + L.off_tmp);
-    {
-        long long nb = (d->nrows + 255) / 256;
-        if (nb > capb) nb = capb;
-        if (nb < 1) nb = 1;
-        k_cand_sizes<<<(unsigned)nb, 256, 0, st>>>(cand, cnt, tc1, d->nrows, d->ncols,
-                                                   d->set_diag ? 1 : 0,
-                                                   candptr);
-        CK(cudaGetLastError());
-        CK(cudaMemsetAsync(candptr + d->nrows, 0, sizeof(long long), st));
-        s = scan_exclusive(candptr, n1, scan, st);
-        if (s != OP2G_OK) return s;
-    }
-    int cap = hm.max_cand > 1 ? hm.max_cand : 1;
-    CK(cudaMemcpyAsync(&misc->cap, &cap, sizeof(int), cudaMemcpyHostToDevice, st));
-    s = sp_rows_launch(S, pd, simple, cnt, tlist, cap, candptr, tmp, (long long *)rowptr, st);
-    if (s != OP2G_OK) return s;
-    CK(cudaMemsetAsync(rowptr + d->nrows, 0, sizeof(long long), st));
-    s = scan_exclusive((long long *)rowptr, n1, scan, st);
-    if (s != OP2G_OK) return s;
-    long long total = 0;
-    int err = 0;
-    CK(cudaMemcpyAsync(&total, rowptr + d->nrows, sizeof total, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&err, &misc->err, sizeof err, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    if (err & OP2G_DEVERR_MAP_BOUNDS)
-        return op2g::fail(OP2G_ERR_BOUNDS, "a map value is outside the row or column set");
-    if (err & OP2G_DEVERR_CAPACITY)
+    if (hm.err & OP2G_DEVERR_CAPACITY)
         return op2g::fail(OP2G_ERR_CAPACITY, "sparsity row candidate capacity exceeded");
-    if (nnz) *nnz = total;
+    // any non-zero byte pattern means "yes"
+    CK(cudaMemsetAsync(&misc->done, 1, sizeof(int), st));
+    if (hm.small) CK(cudaMemsetAsync(&misc->small, 1, sizeof(int), st));
+    if (nnz) *nnz = hm.total;
     return OP2G_OK;
 }
 
@@ -661,15 +1200,22 @@ op2g_status op2g_sparsity_fill(const op2g_sparsity_desc *d, void *ws, size_t ws_
     cudaStream_t st = (cudaStream_t)stream;
     char *w = (char *)ws;
     SpMisc *misc = (SpMisc *)(w + L.off_misc);
-    const long long *candptr = (const long long *)(w + L.off_candptr);
     const int *tmp = (const int *)(w + L.off_tmp);
-    int cap = 0;
-    CK(cudaMemcpyAsync(&cap, &misc->cap, sizeof cap, cudaMemcpyDeviceToHost, st));
+    SpMisc hm;
+    CK(cudaMemcpyAsync(&hm, misc, sizeof hm, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (cap < 1) return op2g::fail(OP2G_ERR_INVALID, "op2g_sparsity_fill before op2g_sparsity_count");
+    if (!hm.done) return op2g::fail(OP2G_ERR_INVALID, "op2g_sparsity_fill before op2g_sparsity_count");
     if (d->nrows == 0) return OP2G_OK;
-    k_rows_copy<<<grid_for_rows(d->nrows), 256, 0, st>>>(d->nrows, candptr, tmp,
-                                                         (const long long *)rowptr, colidx);
+    if (hm.small) {
+        const int rb = rows_per_batch(d->nrows);
+        const long long nb = (d->nrows + rb * 8ll - 1) / (rb * 8ll);
+        k_batches_copy<<<(unsigned)nb, 256, 0, st>>>(d->nrows, (const long long *)(w + L.off_ptr),
+                                                     L.tc, d->set_diag, rb, tmp,
+                                                     (const long long *)rowptr, colidx);
+    } else {
+        k_rows_copy<<<grid_for_rows(d->nrows), 256, 0, st>>>(
+            d->nrows, (const long long *)(w + L.off_candptr), tmp, (const long long *)rowptr, colidx);
+    }
     CK(cudaGetLastError());
     return OP2G_OK;
 }
