@@ -261,7 +261,9 @@ typedef struct op2g_launch_desc {
 
 /* Launch the wrapper over [start, end) on `stream`.  Asynchronous. */
 op2g_status op2g_kernel_launch(op2g_kernel *k, const op2g_launch_desc *d, void *stream);
-/* The launch shape op2g_kernel_launch uses (pure function, no device use):
+/* The launch shape op2g_kernel_launch starts from (pure function, no device
+ * use; for grid == 0 a launch splits the CTAs of register-heavy wrappers into
+ * ones of 64 threads and lifts the cap for loops that insert into a Mat):
  * `items` iterations over `entities` entities, a wrapper compiled for
  * `block_size` threads holding `ctas_per_sm` CTAs on each of `sms` SMs,
  * the descriptor's `grid` request, and whether the wrapper has the balanced

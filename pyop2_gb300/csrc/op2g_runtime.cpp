@@ -11,6 +11,7 @@
 #include <cuda_runtime_api.h>
 #include <nvrtc.h>
 
+#include <algorithm>
 #include <cerrno>
 #include <cstdint>
 #include <cstdio>
@@ -209,11 +210,14 @@ op2g_status build_cubin(const std::string &src, const std::string &arch, const c
     return OP2G_OK;
 }
 
+constexpr int SMALL_CTA = 64;
+
 struct Loaded {
     CUmodule mod = nullptr;
     CUfunction f = nullptr, fb = nullptr, fc = nullptr;  // plain, batched, chunked
     int regs = -1;
     int occ = 0;  // resident CTAs per SM
+    int occ_small = 0;  // the same for CTAs of SMALL_CTA threads
     int sms = 0;
     // staged wrappers: dynamic shared memory the function is set up for, and
     // the resident CTAs per SM at the last size asked for
@@ -252,6 +256,9 @@ op2g_status load_module(const std::string &cubin, const char *fname, const char 
     D.FuncGetAttribute(&L.regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.f);
     if (D.OccupancyMaxActiveBlocksPerMultiprocessor(&L.occ, L.f, bs, 0) != CUDA_SUCCESS) L.occ = 1;
     if (L.occ < 1) L.occ = 1;
+    if (bs > SMALL_CTA && D.OccupancyMaxActiveBlocksPerMultiprocessor(
+                              &L.occ_small, L.f, SMALL_CTA, 0) != CUDA_SUCCESS)
+        L.occ_small = 0;
     cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev);
     if (L.sms < 1) L.sms = 1;
     auto res = per_dev.emplace(dev, L);
@@ -303,6 +310,51 @@ static bool use_aligned(const op2g_kernel *k, const op2g_launch_desc *d) {
     for (const auto &sa : k->al_args)
         if ((uintptr_t)d->ptrs[sa.first] % (uintptr_t)sa.second) return false;
     return true;
+}
+
+// What a default launch changes about op2g_launch_shape's answer, knowing the
+// compiled wrapper.
+//
+// Heavy wrappers (an element kernel whose registers leave at most 1,280
+// threads per SM) issue FP64 most of the time, so what costs is an SM that
+// still works while the others have nothing left.  They run as CTAs of 64
+// threads where those keep more threads resident than the compiled size (190
+// registers: 5 x 64 against 1 x 256), or where the launch is only a few waves
+// long.  Measured at 262,144 prisms: elasticity VJP (190 registers) 2.48 ->
+// 2.21 ms, action (128) 1.45 -> 1.43 ms; at 1.57 M tets the nonlinear residual
+// 0.226 -> 0.223 ms.  Light wrappers keep large CTAs: launching one costs the
+// GPU about 1.2 ns, which a copy of 12.6 M values in CTAs of 64 would feel
+// (0.107 against 0.039 ms, uncapped).
+//
+// Loops that insert into a Mat run one CTA per block of iterations, without
+// the cap of 4 waves: their iterations are long enough, and CTAs that start
+// when another ends even out the SMs (P1 tet assembly, 6 M cells: 0.965 ->
+// 0.936 ms).
+static void refine_shape(const Loaded &L, const Signature &S, int64_t items, int32_t *grid,
+                         int32_t *bs, int32_t *chunked) {
+    if (!L.fc || L.occ_small < 1) return;   // shared-memory tables, or small CTAs already
+    const int64_t resident = (int64_t)L.occ * S.block_size;
+    bool mat = false;
+    for (const ArgInfo &A : S.args) mat = mat || A.d.kind == OP2G_ARG_MAT;
+    bool use = resident <= 1280 && ((int64_t)L.occ_small * SMALL_CTA > resident || resident <= 512 ||
+                                    items < 8 * resident * L.sms);
+    // The balanced entry stays where its CTAs are all on the SMs at once, and
+    // where small CTAs would leave a few of them for a second round that takes
+    // as long as an iteration alone (79,380 prisms on 77,824 resident threads,
+    // action: 0.492 against 0.536 ms; assembly gains all the same, 1.60 -> 1.30).
+    const int64_t round = (int64_t)L.occ_small * SMALL_CTA * L.sms;
+    if (*chunked && (*grid <= (int64_t)L.occ * L.sms ||
+                     (!mat && items > round && items < round + round / 7)))
+        return;
+    if (!use) {
+        if (mat && !*chunked)
+            *grid = (int32_t)std::min<int64_t>((items + *bs - 1) / *bs, INT32_MAX);
+        return;
+    }
+    const int64_t need = (items + SMALL_CTA - 1) / SMALL_CTA, cap = 8ll * L.occ_small * L.sms;
+    *grid = (int32_t)std::min<int64_t>(mat || need < cap ? need : cap, INT32_MAX);
+    *bs = SMALL_CTA;
+    *chunked = 0;
 }
 
 extern "C" {
@@ -591,6 +643,7 @@ op2g_status op2g_kernel_launch(op2g_kernel *k, const op2g_launch_desc *d, void *
     op2g_launch_shape((items + cpt - 1) / cpt, (d->end - d->start + cpt - 1) / cpt,
                       k->sig.block_size, L->sms, L->occ, d->grid, L->fc != nullptr, &grid, &bs,
                       &chunked);
+    if (d->grid == 0) refine_shape(*L, k->sig, (items + cpt - 1) / cpt, &grid, &bs, &chunked);
     void *params[] = {buf};
     return launch(chunked ? L->fc : L->f, (unsigned)grid, (unsigned)bs, params, stream);
 }
