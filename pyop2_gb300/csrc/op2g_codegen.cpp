@@ -227,6 +227,8 @@ struct Gen {
     int cells_per_thread = 1;  // what the sweep loop was generated with
     // The variant for aligned direct arguments (aligned_direct_args).
     bool align_hints = false;
+    // Elements a thread of a pure reduction loads together, 0 for other loops.
+    int red_unroll = 0;
 
     explicit Gen(const Signature &s) : S(s) {
         nf = (S.loop.extruded && S.loop.iteration_region == OP2G_ON_INTERIOR_FACETS) ? 2 : 1;
@@ -785,9 +787,35 @@ struct Gen {
         O << "    __syncthreads();\n";
         O << "    return;\n";
         O << "  }\n";
-        emit_global_reductions();
+        emit_global_reductions(true);
         O << "}\n\n";
         staging = false;
+    }
+
+    // A pure reduction: a flat loop over a whole set whose arguments are
+    // Globals and direct READ Dats of a few bytes per entity.  Its threads
+    // load the rows of several iterations (up to 64 bytes) before the first
+    // kernel call, which then reads registers: with a row at a time a thread
+    // keeps one load in flight, and any branch in the kernel or the reduction
+    // waits for it.  With one resident wave of threads instead of four, 12.6 M
+    // floats, sum / min / max: 29 -> 21 us, doubles 120 -> 85 us (FP64-bound:
+    // a compare costs the pipe as much as an FMA, and both the kernel and the
+    // accumulator compare; ordering the doubles by their bits on the integer
+    // pipe instead took 132 us).  Returns the iterations loaded together.
+    int reduction_unroll() const {
+        if (S.loop.extruded || S.loop.indexed || S.loop.prefetch || S.loop.cells_per_thread > 1 ||
+            S.loop.pass_layer_arg || !S.loop.nc_reads || any_staged)
+            return 0;
+        long long bytes = 0;
+        for (const ArgInfo &A : S.args) {
+            if (A.d.kind == OP2G_ARG_GLOBAL) continue;
+            if (A.d.kind != OP2G_ARG_DAT || A.d.map >= 0 || A.d.access != OP2G_READ ||
+                A.d.group != 0 || A.d.dim > 4 || elt_size(A.d.dtype) < 4)
+                return 0;
+            bytes += A.d.dim * (long long)elt_size(A.d.dtype);
+        }
+        if (bytes == 0 || bytes > 32) return 0;
+        return bytes <= 8 ? 8 : (int)(64 / bytes);
     }
 
     // Per-thread accumulators of Global INC/MIN/MAX arguments.
@@ -809,25 +837,73 @@ struct Gen {
         }
     }
 
-    // Warp-reduced Global results, one atomic per warp (pyop2/parloop.py:
-    // 409-452 semantics on one device: INC goes to the zeroed temporary,
-    // MIN/MAX straight into the Global).
-    void emit_global_reductions() {
+    // Reduced Global results (pyop2/parloop.py:409-452 semantics on one
+    // device: INC goes to the zeroed temporary, MIN/MAX straight into the
+    // Global): each warp reduces by shuffles, the CTA's first warp reduces
+    // the warps' results from shared memory and issues one atomic per
+    // component.  All CTAs hit the same few addresses, which the L2 serves
+    // one at a time: with an atomic per warp, the 38,912 warps of a 12.6 M-
+    // element float sum / min / max took 70 us, with one per CTA 29.
+    // Few warps (small launches, and each work item of a batched launch, whose
+    // loops have Globals of their own) go straight to the atomics, without the
+    // barriers; so do loops of more than RED_MAX components (shared memory).
+    // Few means more for loops through maps, whose warps end far enough apart
+    // (320,000 triangles, action and area: 42 us either way at 10,000 warps
+    // with their own atomics, 43 with the barriers).
+    static constexpr int RED_MAX = 16, RED_WARPS = 2048, RED_WARPS_MAPS = 32768;
+
+    // staged_run: a staged wrapper's own run function, launched alone.
+    void emit_global_reductions(bool staged_run = false) {
         std::ostringstream &O = o;
+        int comps = 0;
+        for (const ArgInfo &A : S.args)
+            if (A.d.kind == OP2G_ARG_GLOBAL && A.d.access != OP2G_READ) comps += A.d.dim;
+        if (!comps) return;
+        auto reduce = [](int access) {
+            return access == OP2G_INC ? "warp_sum" : access == OP2G_MIN ? "warp_min" : "warp_max";
+        };
+        auto atomic = [](int access) {
+            return access == OP2G_INC ? "atomic_inc"
+                   : access == OP2G_MIN ? "atomic_min" : "atomic_max";
+        };
+        const int W = S.block_size / 32;
+        const bool cta = comps <= RED_MAX && W > 1;
+        if (cta)
+            O << "  const bool cta_ = " << (staged_run ? "" : "alone && ")
+              << "(long long)gridDim.x * (blockDim.x >> 5) > "
+              << (S.maps.empty() ? RED_WARPS : RED_WARPS_MAPS) << ";\n";
         for (size_t a = 0; a < S.args.size(); ++a) {
             const ArgInfo &A = S.args[a];
             if (A.d.kind != OP2G_ARG_GLOBAL || A.d.access == OP2G_READ) continue;
             const char *T = ctype_of(A.d.dtype);
-            const char *red = A.d.access == OP2G_INC ? "warp_sum"
-                              : A.d.access == OP2G_MIN ? "warp_min" : "warp_max";
-            const char *atom = A.d.access == OP2G_INC ? "atomic_inc"
-                               : A.d.access == OP2G_MIN ? "atomic_min" : "atomic_max";
+            if (cta) O << "  __shared__ " << T << " sred" << a << "_[" << A.d.dim << "][" << W << "];\n";
             O << "  for (int j = 0; j < " << A.d.dim << "; ++j) {\n";
-            O << "    " << T << " v_ = op2g::" << red << "(gacc" << a << "[j]);\n";
-            O << "    if ((threadIdx.x & 31) == 0) op2g::" << atom << "(((" << T << " *)p.ptr["
-              << A.slot << "]) + j, v_);\n";
+            O << "    " << T << " v_ = op2g::" << reduce(A.d.access) << "(gacc" << a << "[j]);\n";
+            O << "    if ((threadIdx.x & 31) == 0) {\n";
+            if (cta) O << "      if (cta_) sred" << a << "_[j][threadIdx.x >> 5] = v_; else\n";
+            O << "      op2g::" << atomic(A.d.access) << "(((" << T << " *)p.ptr[" << A.slot
+              << "]) + j, v_);\n    }\n";
             O << "  }\n";
         }
+        if (!cta) return;
+        O << "  if (!cta_) return;\n";
+        O << "  __syncthreads();\n";
+        O << "  if (threadIdx.x < 32) {\n";
+        O << "    const int nw_ = blockDim.x >> 5, w_ = threadIdx.x < nw_ ? threadIdx.x : 0;\n";
+        for (size_t a = 0; a < S.args.size(); ++a) {
+            const ArgInfo &A = S.args[a];
+            if (A.d.kind != OP2G_ARG_GLOBAL || A.d.access == OP2G_READ) continue;
+            const char *T = ctype_of(A.d.dtype);
+            O << "    for (int j = 0; j < " << A.d.dim << "; ++j) {\n";
+            O << "      " << T << " v_ = sred" << a << "_[j][w_];\n";
+            if (A.d.access == OP2G_INC)   // lanes without a warp add nothing
+                O << "      if (threadIdx.x >= nw_) v_ = " << inc_zero(A.d.dtype) << ";\n";
+            O << "      v_ = op2g::" << reduce(A.d.access) << "(v_);\n";
+            O << "      if (threadIdx.x == 0) op2g::" << atomic(A.d.access) << "(((" << T
+              << " *)p.ptr[" << A.slot << "]) + j, v_);\n";
+            O << "    }\n";
+        }
+        O << "  }\n";
     }
 
     std::string emit() {
@@ -886,7 +962,7 @@ struct Gen {
 
         // ----- the run function: a strided sweep of [start, end) plus reductions
         O << "__device__ __forceinline__ void op2g_run(const op2g_params_t &p, long long start, "
-             "long long end, long long first, long long stride) {\n";
+             "long long end, long long first, long long stride, bool alone) {\n";
         emit_global_init();
         if (extr) {
             // pyop2/codegen/builder.py:771-812 (layer extents per iteration region)
@@ -957,8 +1033,30 @@ struct Gen {
                          !direct_update && !has_pass)
                             ? S.loop.cells_per_thread
                             : 1;
-        cells_per_thread = cpt;
-        if (cpt > 1) {
+        red_unroll = reduction_unroll();
+        cells_per_thread = red_unroll ? red_unroll : cpt;
+        if (red_unroll) {
+            O << "  for (long long base_ = i0_ + first; base_ < i1_; base_ += stride * " << red_unroll
+              << ") {\n";
+            for (size_t a = 0; a < S.args.size(); ++a)
+                if (S.args[a].d.kind == OP2G_ARG_DAT)
+                    O << "   " << ctype_of(S.args[a].d.dtype) << " rd" << a << "_[" << red_unroll << "]["
+                      << S.args[a].d.dim << "];\n";
+            O << "#pragma unroll\n   for (int c_ = 0; c_ < " << red_unroll << "; ++c_) {\n"
+              << "    const long long ic_ = base_ + c_ * stride + threadIdx.x;\n"
+              << "    if (ic_ < i1_) {\n";
+            for (size_t a = 0; a < S.args.size(); ++a) {
+                const op2g_arg_desc &d = S.args[a].d;
+                if (d.kind != OP2G_ARG_DAT) continue;
+                O << "#pragma unroll\n     for (int j = 0; j < " << d.dim << "; ++j) rd" << a
+                  << "_[c_][j] = __ldg((const " << ctype_of(d.dtype) << " *)p.ptr[" << S.args[a].slot
+                  << "] + ic_ * " << gstride(a) << " + j);\n";
+            }
+            O << "    }\n   }\n";
+            O << "#pragma unroll\n   for (int c_ = 0; c_ < " << red_unroll << "; ++c_) {\n"
+              << "    const long long it = base_ + c_ * stride + threadIdx.x;\n"
+              << "    const bool active = it < i1_;\n";
+        } else if (cpt > 1) {
             guard_unpack = true;
             O << "  for (long long base_ = i0_ + first; base_ < i1_; base_ += stride * " << cpt << ") {\n";
             O << "#pragma unroll\n";
@@ -1028,7 +1126,7 @@ struct Gen {
             // cannot prove them distinct), so each thread would otherwise
             // keep one load in flight (a 12.58 M-cell direct copy: 0.042 ->
             // 0.037 ms; a prefetch is a hint, nothing it reads is used).
-            if (!S.loop.indexed && cpt == 1 && !staging) {
+            if (!S.loop.indexed && cpt == 1 && !staging && !red_unroll) {
                 bool any = false;
                 for (size_t a = 0; a < S.args.size(); ++a) {
                     const op2g_arg_desc &d = S.args[a].d;
@@ -1091,7 +1189,7 @@ struct Gen {
             O << "    __syncthreads();\n";
             O << "    par_ ^= 1;\n";
         }
-        if (cpt > 1) O << "   }\n";  // cells of the step
+        if (cpt > 1 || red_unroll) O << "   }\n";  // cells of the step
         O << "  }\n";  // sweep loop
         guard_unpack = false;
         emit_global_reductions();
@@ -1111,7 +1209,7 @@ struct Gen {
             O << "extern \"C\" __global__ void __launch_bounds__(" << BS
               << ") op2g_wrap(const __grid_constant__ op2g_params_t p) {\n"
               << "  op2g_run(p, p.start, p.end, (long long)blockIdx.x * " << bdim
-              << ", (long long)gridDim.x * " << bdim << ");\n}\n";
+              << ", (long long)gridDim.x * " << bdim << ", true);\n}\n";
         }
         if (!any_shared && !any_staged) {
             // Balanced form for launches of a few CTAs per SM: CTA b takes the
@@ -1123,14 +1221,14 @@ struct Gen {
               << "  const long long c_ = (n_ + gridDim.x - 1) / gridDim.x;\n"
               << "  const long long s_ = p.start + (long long)blockIdx.x * c_;\n"
               << "  const long long e_ = s_ + c_ < p.end ? s_ + c_ : p.end;\n"
-              << "  if (s_ < e_) op2g_run(p, s_, e_, 0, (long long)blockDim.x);\n}\n";
+              << "  if (s_ < e_) op2g_run(p, s_, e_, 0, (long long)blockDim.x, true);\n}\n";
         }
         O << "extern \"C\" __global__ void __launch_bounds__(" << BS
           << ") op2g_wrap_batched(const op2g_params_t *__restrict__ P, const long long "
              "*__restrict__ work, long long nwork) {\n"
           << "  for (long long w = blockIdx.x; w < nwork; w += gridDim.x) {\n"
           << "    const op2g_params_t &p = P[work[3 * w]];\n"
-          << "    op2g_run(p, work[3 * w + 1], work[3 * w + 2], 0, " << BS << ");\n"
+          << "    op2g_run(p, work[3 * w + 1], work[3 * w + 2], 0, " << BS << ", false);\n"
           << "  }\n}\n";
         return O.str();
     }
@@ -1208,7 +1306,9 @@ struct Gen {
                     // direct: pointer into the Dat (pyop2/codegen/builder.py:367-377);
                     // in a staged wrapper a fetched READ argument is read from
                     // its partition buffer in shared memory
-                    if (staging && st_dir[a])
+                    if (red_unroll)
+                        kargs.push_back("op2g::ptr(rd" + an + "_[c_])");
+                    else if (staging && st_dir[a])
                         kargs.push_back("op2g::ptr((" + std::string(T) + " *)dv" + an +
                                         "[vb_] + (n - c0_) * " + std::to_string(A.d.dim) + ")");
                     else {
@@ -1549,6 +1649,8 @@ std::vector<std::pair<int, int>> aligned_direct_args(const Signature &S) {
     }
     return out;
 }
+
+int reduction_unroll(const Signature &S) { return Gen(S).reduction_unroll(); }
 
 std::string generate_source(const Signature &S, int *cells_per_thread, bool align_hints) {
     Gen g(S);

@@ -46,6 +46,8 @@ std::string validate_signature(const Signature &S);
 // launched only when their pointers are).
 std::string generate_source(const Signature &S, int *cells_per_thread = nullptr,
                             bool align_hints = false);
+// Iterations a thread of a pure reduction loads together, 0 for other loops.
+int reduction_unroll(const Signature &S);
 // Direct Dat arguments whose rows are a multiple of 16 bytes, as (pointer
 // slot, row alignment in bytes: 16 or 32); empty for staged wrappers.
 std::vector<std::pair<int, int>> aligned_direct_args(const Signature &S);

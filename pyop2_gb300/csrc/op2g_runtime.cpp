@@ -296,6 +296,7 @@ struct op2g_kernel {
     int param_bytes = 0;
     bool staged = false;   // the wrapper stages arguments on a plan (OP2G_SCATTER_STAGED)
     int cells_per_thread = 1;
+    bool reduction = false;   // a pure reduction (reduction_unroll)
     // Direct arguments with rows of a multiple of 16 bytes (pointer slot,
     // alignment): a second variant of the wrapper declares their rows
     // aligned, and a launch runs it when every such pointer is aligned.
@@ -437,6 +438,7 @@ op2g_status op2g_kernel_create(const char *user_src, const char *kernel_name,
     op2g_kernel *k = new op2g_kernel();
     k->sig = S;
     k->source = generate_source(S, &k->cells_per_thread);
+    k->reduction = reduction_unroll(S) > 0;
     k->param_bytes = 8 * (5 + (S.nptrs > 0 ? S.nptrs : 1) + (nmaps > 0 ? nmaps : 1));
     for (int r : staged_args(S))
         if (r >= 0) k->staged = true;
@@ -643,7 +645,11 @@ op2g_status op2g_kernel_launch(op2g_kernel *k, const op2g_launch_desc *d, void *
     op2g_launch_shape((items + cpt - 1) / cpt, (d->end - d->start + cpt - 1) / cpt,
                       k->sig.block_size, L->sms, L->occ, d->grid, L->fc != nullptr, &grid, &bs,
                       &chunked);
-    if (d->grid == 0) refine_shape(*L, k->sig, (items + cpt - 1) / cpt, &grid, &bs, &chunked);
+    // A pure reduction runs one resident wave: its threads keep accumulators,
+    // and fewer of them settle sooner and reduce into fewer atomics.
+    if (d->grid == 0 && k->reduction && !chunked)
+        grid = (int32_t)std::min<int64_t>(grid, (int64_t)L->occ * L->sms);
+    else if (d->grid == 0) refine_shape(*L, k->sig, (items + cpt - 1) / cpt, &grid, &bs, &chunked);
     void *params[] = {buf};
     return launch(chunked ? L->fc : L->f, (unsigned)grid, (unsigned)bs, params, stream);
 }
