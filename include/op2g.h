@@ -426,6 +426,19 @@ op2g_status op2g_colour_noalloc(int64_t ncells, int32_t nmaps, const int32_t *co
                                 int32_t max_colours, int32_t *colour, int32_t *order,
                                 int64_t *colour_ptr, int32_t *ncolours, void *stream);
 
+/* ------------------------------------------------ pointwise linear algebra
+ * Dat arithmetic (pyop2/types/dat.py:343-574) on the owned values as flat
+ * arrays of n elements of a 32- or 64-bit type (others: OP2G_ERR_UNSUPPORTED). */
+enum { OP2G_VEC_ADD = 0, OP2G_VEC_SUB = 1, OP2G_VEC_MUL = 2, OP2G_VEC_DIV = 3, OP2G_VEC_NEG = 4 };
+/* out[i] = a[i] op b[i], or op *scalar (host, read during the call) when b is
+ * NULL; OP2G_VEC_NEG takes neither.  out may be a or b.  Asynchronous. */
+op2g_status op2g_vec_op(int32_t op, int32_t dtype, int64_t n, const void *a, const void *b,
+                        const void *scalar, void *out, void *stream);
+/* *result (host, one element of the type) = sum a[i] b[i], accumulated in the
+ * type in an order fixed by n and the arrays' alignment.  Waits for `stream`. */
+op2g_status op2g_vec_dot(int32_t dtype, int64_t n, const void *a, const void *b, void *result,
+                         void *stream);
+
 /* --------------------------------------------------------- measurement */
 /* Time a register-resident FP64 FMA loop over the whole GPU and return the
  * achieved FP64 rate (flop/s, FMA = 2) -- the second roofline ceiling of the

@@ -120,12 +120,16 @@ SIGNATURES = {
                            _p, ctypes.c_size_t, _p, _p, _p, _pi32, _p]),
     "op2g_colour_noalloc": (_i32, [_i64, _i32, ctypes.POINTER(_p), _pi32, ctypes.POINTER(_i64),
                                    _i32, _p, _p, _p, _pi32, _p]),
+    "op2g_vec_op": (_i32, [_i32, _i32, _i64, _p, _p, _p, _p, _p]),
+    "op2g_vec_dot": (_i32, [_i32, _i64, _p, _p, _p, _p]),
     "op2g_probe_fp64_peak": (_i32, [ctypes.POINTER(ctypes.c_double), _p]),
     "op2g_stage_plan_workspace": (_i32, [_i64, _i32, _i64, ctypes.POINTER(ctypes.c_size_t)]),
     "op2g_stage_plan_count": (_i32, [_i64, _i32, _p, _i64, _p, ctypes.c_size_t, _p, _p,
                                      ctypes.POINTER(_i64), _pi32, _p]),
     "op2g_stage_plan_fill": (_i32, [_i64, _i32, _p, _i64, _p, _p, _p, _p, _p]),
 }
+
+VEC_ADD, VEC_SUB, VEC_MUL, VEC_DIV, VEC_NEG = range(5)
 
 _lib = None
 

@@ -8,14 +8,20 @@ back once.
 """
 import numpy as np
 
+from pyop2_gb300 import _lib, device
 from pyop2_gb300 import exceptions as ex
 from pyop2_gb300 import utils
 from pyop2_gb300.configuration import configuration
-from pyop2_gb300.datatypes import ScalarType
+from pyop2_gb300.datatypes import ScalarType, as_code
 from pyop2_gb300.device import Mirror
 from pyop2_gb300.types.access import Access
 from pyop2_gb300.types.dataset import DataSet
 from pyop2_gb300.types.set import ExtrudedSet, Set
+
+
+# element types of the library's vector kernels
+_VEC_CODES = {np.dtype(t): as_code(np.dtype(t)) for t in
+              ("float64", "float32", "int32", "uint32", "int64", "uint64")}
 
 
 class DataCarrier:
@@ -205,7 +211,6 @@ class Dat(AbstractDat):
         """A Dat whose device storage is ``tensor`` (CUDA, contiguous, matching
         shape and dtype), without copying.  The Dat writes into the tensor."""
         import torch
-        from pyop2_gb300 import device
         if type(dataset) is Set:
             dataset = dataset ** 1
         d = cls.__new__(cls)
@@ -274,10 +279,68 @@ class Dat(AbstractDat):
             filename = filename + ".npy"
         self.data[:] = np.load(filename)
 
-    # ---- pointwise linear algebra (pyop2/types/dat.py:343-574), executed
-    # as generated direct par_loops over the owned entities, as the
-    # reference does
+    # ---- pointwise linear algebra (pyop2/types/dat.py:343-574) over the
+    # owned entities: operands of one 32- or 64-bit type run the library's
+    # vector kernels (op2g_vec_op, op2g_vec_dot), anything else a generated
+    # direct par_loop, as the reference does
     _kernel_cache = {}
+    _VEC_OPS = {"add": _lib.VEC_ADD, "sub": _lib.VEC_SUB, "mul": _lib.VEC_MUL,
+                "div": _lib.VEC_DIV}
+
+    def _vec_code(self, other):
+        """Element type code when the vector kernels apply to self and other
+        (a Dat, or a number), else None.  Views, Dats of other sets or with
+        frozen halos, and loops that are checked or timed one by one take the
+        par_loop, with its checks and errors."""
+        code = _VEC_CODES.get(self._dtype)
+        if code is None or type(self) is not Dat or self._halo_frozen or \
+                configuration["debug"] or configuration["profiling"]:
+            return None
+        if type(other) is Dat:
+            if other._dtype != self._dtype or other._halo_frozen or \
+                    other._dataset.set is not self._dataset.set:
+                return None
+            self._check_shape(other)
+        elif not isinstance(other, (int, float, np.number)):
+            return None
+        return code
+
+    def _vec_run(self, op, code, other, out):
+        """out = self op other, other a Dat or a number (None for -self)."""
+        device.require()
+        a = self._device_ptr()
+        o = a if out is self else out._device_ptr()
+        b = s = None
+        if isinstance(other, Dat):
+            b = other._device_ptr()
+        elif type(other) is float and code == _lib.F64:
+            v = _lib.ctypes.c_double(other)
+            s = _lib.ctypes.byref(v)
+        elif other is not None:     # the conversion a Global of this type makes
+            v = utils.verify_reshape(other, self._dtype, (1,))
+            s = v.ctypes.data
+        _lib.check(_lib.lib().op2g_vec_op(op, code, self._dataset.size * self._dataset.cdim, a, b,
+                                          s, o, device.stream_handle()))
+        out._m.dev_modified()
+        out.increment_dat_version()
+        out.halo_valid = False
+
+    def _new_like(self):
+        """A Dat for a result on this one's dataset.  Its owned values are
+        written next, so they need clearing only when there are ghosts."""
+        d = Dat.__new__(Dat)
+        ds = d._dataset = self._dataset
+        d.comm = ds.comm
+        d._shape = self._shape
+        d._dtype = self._dtype
+        m = d._m = Mirror(self._dtype, self._shape)
+        if ds.size == ds.total_size:
+            m._dev = device.empty_bytes(m.nbytes)
+            m.state = "device"
+        d._name = "dat_#x%x" % id(d)
+        d.halo_valid = True
+        d._version = 0
+        return d
 
     def _kernel(self, key, body, name):
         from pyop2_gb300.local_kernel import Kernel
@@ -299,6 +362,11 @@ class Dat(AbstractDat):
                              % (self.dataset.dim, other.dataset.dim))
 
     def _op(self, other, op, opname):
+        code = self._vec_code(other)
+        if code is not None:
+            ret = self._new_like()
+            self._vec_run(self._VEC_OPS[opname], code, other, ret)
+            return ret
         from pyop2_gb300.datatypes import as_cstr
         from pyop2_gb300.parloop import run_once as par_loop
         from pyop2_gb300.types.access import READ, WRITE
@@ -314,6 +382,10 @@ class Dat(AbstractDat):
         return ret
 
     def _iop(self, other, op, opname):
+        code = self._vec_code(other)
+        if code is not None:
+            self._vec_run(self._VEC_OPS[opname], code, other, self)
+            return self
         from pyop2_gb300.datatypes import as_cstr
         from pyop2_gb300.parloop import run_once as par_loop
         from pyop2_gb300.types.access import READ, RW
@@ -368,6 +440,11 @@ class Dat(AbstractDat):
         return Dat(self)
 
     def __neg__(self):
+        code = self._vec_code(self)
+        if code is not None:
+            ret = self._new_like()
+            self._vec_run(_lib.VEC_NEG, code, None, ret)
+            return ret
         from pyop2_gb300.datatypes import as_cstr
         from pyop2_gb300.parloop import run_once as par_loop
         from pyop2_gb300.types.access import READ, WRITE
@@ -381,8 +458,16 @@ class Dat(AbstractDat):
         return ret
 
     def inner(self, other):
-        """Euclidean inner product over the owned entities (a Global INC
-        reduction on the device)."""
+        """Euclidean inner product over the owned entities, reduced on the
+        device."""
+        code = self._vec_code(other) if isinstance(other, Dat) else None
+        if code is not None:
+            device.require()
+            out = np.empty(1, dtype=self._dtype)
+            _lib.check(_lib.lib().op2g_vec_dot(code, self._dataset.size * self._dataset.cdim,
+                                               self._device_ptr(), other._device_ptr(),
+                                               out.ctypes.data, device.stream_handle()))
+            return out[0]
         from pyop2_gb300.datatypes import as_cstr
         from pyop2_gb300.parloop import run_once as par_loop
         from pyop2_gb300.types.access import INC, READ
