@@ -7,6 +7,7 @@ historical OP2 CUDA backend (doc/sphinx/source/backends.rst:222-236): the host
 copy is refreshed only when the host reads data that the device modified, and
 uploaded only when a launch needs data that the host modified.
 """
+import math
 import warnings
 
 import numpy as np
@@ -45,9 +46,16 @@ def require():
     _ready = True
 
 
+_device = None      # (ordinal, torch.device) of the last call
+
+
 def device():
+    global _device
     require()
-    return torch.device("cuda", configuration["device"])
+    n = configuration["device"]
+    if _device is None or _device[0] != n:
+        _device = (n, torch.device("cuda", n))
+    return _device[1]
 
 
 def sm_count():
@@ -79,8 +87,11 @@ if hasattr(torch, "uint16"):
     _TORCH["uint16"] = torch.uint16
 
 
+_TORCH_OF = {np.dtype(name): t for name, t in _TORCH.items()}
+
+
 def torch_dtype(dtype):
-    return _TORCH[np.dtype(dtype).name]
+    return _TORCH_OF[np.dtype(dtype)]
 
 
 def empty_bytes(nbytes):
@@ -135,13 +146,13 @@ class Mirror:
     def __init__(self, dtype, shape, data=None):
         self.dtype = np.dtype(dtype)
         self.shape = tuple(shape)
+        # worked out once: these run for every access of every loop's data
+        self.size = math.prod(self.shape)
+        self.nbytes = self.size * self.dtype.itemsize
+        self._typed = (None, None)  # device buffer and its shaped view
         self._host = data           # numpy array or None (= zeros)
         self._dev = None            # torch uint8 tensor or None
         self.state = "host"
-
-    @property
-    def nbytes(self):
-        return int(np.prod(self.shape)) * self.dtype.itemsize
 
     # ---- host side
     def host(self, write):
@@ -181,11 +192,35 @@ class Mirror:
         self.state = "device"
 
     def tensor(self):
-        """Typed device view (shape-flattened) of the current data."""
+        """Typed device view (flat) of the current data."""
+        return self.shaped().view(-1)
+
+    def shaped(self):
+        """Typed device view of the current data in the mirror's shape.  The
+        view of a buffer is made once; each call returns an alias of it, so
+        that what a caller does to its tensor object stays with the caller."""
         b = self.dev()
-        n = self.nbytes
-        return b[:n].view(torch_dtype(self.dtype)) if n else \
-            torch.empty(0, dtype=torch_dtype(self.dtype), device=b.device)
+        src, t = self._typed
+        if src is not b:
+            n, dt = self.nbytes, torch_dtype(self.dtype)
+            t = (b[:n].view(dt) if n else torch.empty(0, dtype=dt, device=b.device)).view(self.shape)
+            self._typed = (b, t)
+        return t.detach()
+
+    def adopt(self, buf):
+        """Make `buf` the device buffer, holding the current data."""
+        self._dev = buf
+        self._typed = (None, None)   # does not keep the old buffer alive
+        self._host = None
+        self.state = "device"
+
+    def overwrite_host(self):
+        """Host array that the caller overwrites in full: marked newer without
+        being read back from the device first."""
+        if self._host is None:
+            self._host = np.empty(self.shape, dtype=self.dtype)
+        self.state = "host"
+        return self._host
 
     def zero(self):
         if self._dev is not None:

@@ -197,7 +197,7 @@ class Dat(AbstractDat):
     def tensor(self):
         """The device values as a torch tensor of shape ``shape`` (no copy).
         Writes through this view must be followed by ``mark_device_modified``."""
-        return self._m.tensor().view(self._shape)
+        return self._m.shaped()
 
     def mark_device_modified(self):
         self._m.dev_modified()
@@ -240,12 +240,9 @@ class Dat(AbstractDat):
         import torch
         if not tensor.is_cuda or not tensor.is_contiguous():
             raise ValueError("_rebind needs a contiguous CUDA tensor")
-        if tensor.numel() != int(np.prod(self._shape)) or \
-                tensor.element_size() != self._dtype.itemsize:
+        if tensor.numel() != self._m.size or tensor.element_size() != self._dtype.itemsize:
             raise ValueError("tensor does not match the Dat's shape and dtype")
-        self._m._dev = tensor.view(-1).view(torch.uint8)
-        self._m._host = None
-        self._m.state = "device"
+        self._m.adopt((tensor if tensor.dim() == 1 else tensor.view(-1)).view(torch.uint8))
         self.increment_dat_version()
 
     # ---- operations
@@ -263,7 +260,13 @@ class Dat(AbstractDat):
         if other is self:
             return
         if subset is None:
-            other.data_with_halos[:] = self.data_ro_with_halos
+            if type(self) is Dat and type(other) is Dat and self._shape == other._shape:
+                # every value is replaced: nothing of the target is read back
+                src = self._m.host(write=False)
+                other.increment_dat_version()
+                other._m.overwrite_host()[...] = src
+            else:
+                other.data_with_halos[:] = self.data_ro_with_halos
             other.halo_valid = True
         elif subset.superset != self.dataset.set:
             raise ex.MapValueError("The subset and dataset are incompatible")
@@ -319,11 +322,19 @@ class Dat(AbstractDat):
         elif other is not None:     # the conversion a Global of this type makes
             v = utils.verify_reshape(other, self._dtype, (1,))
             s = v.ctypes.data
-        _lib.check(_lib.lib().op2g_vec_op(op, code, self._dataset.size * self._dataset.cdim, a, b,
-                                          s, o, device.stream_handle()))
+        _lib.check(_lib.lib().op2g_vec_op(op, code, self._owned()[0], a, b, s, o,
+                                          device.stream_handle()))
         out._m.dev_modified()
         out.increment_dat_version()
         out.halo_valid = False
+
+    def _owned(self):
+        """(owned values, whether there are ghosts), worked out once per DataSet."""
+        ds = self._dataset
+        v = ds.__dict__.get("_owned")
+        if v is None:
+            v = ds.__dict__["_owned"] = (ds.size * ds.cdim, ds.size != ds.total_size)
+        return v
 
     def _new_like(self):
         """A Dat for a result on this one's dataset.  Its owned values are
@@ -334,9 +345,8 @@ class Dat(AbstractDat):
         d._shape = self._shape
         d._dtype = self._dtype
         m = d._m = Mirror(self._dtype, self._shape)
-        if ds.size == ds.total_size:
-            m._dev = device.empty_bytes(m.nbytes)
-            m.state = "device"
+        if not self._owned()[1]:
+            m.adopt(device.empty_bytes(m.nbytes))
         d._name = "dat_#x%x" % id(d)
         d.halo_valid = True
         d._version = 0
@@ -464,9 +474,9 @@ class Dat(AbstractDat):
         if code is not None:
             device.require()
             out = np.empty(1, dtype=self._dtype)
-            _lib.check(_lib.lib().op2g_vec_dot(code, self._dataset.size * self._dataset.cdim,
-                                               self._device_ptr(), other._device_ptr(),
-                                               out.ctypes.data, device.stream_handle()))
+            _lib.check(_lib.lib().op2g_vec_dot(code, self._owned()[0], self._device_ptr(),
+                                               other._device_ptr(), out.ctypes.data,
+                                               device.stream_handle()))
             return out[0]
         from pyop2_gb300.datatypes import as_cstr
         from pyop2_gb300.parloop import run_once as par_loop
