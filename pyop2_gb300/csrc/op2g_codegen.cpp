@@ -229,6 +229,9 @@ struct Gen {
     bool align_hints = false;
     // Elements a thread of a pure reduction loads together, 0 for other loops.
     int red_unroll = 0;
+    // Arguments whose INC contributions neighbouring layers combine
+    // (combines_layers); set while a run function that does so is written.
+    bool layer_pairs = false;
 
     explicit Gen(const Signature &s) : S(s) {
         nf = (S.loop.extruded && S.loop.iteration_region == OP2G_ON_INTERIOR_FACETS) ? 2 : 1;
@@ -576,6 +579,7 @@ struct Gen {
                     if (st_map[r]) need_tg[r] = true;
                 }
         O << "__device__ __forceinline__ void op2g_run_staged(const op2g_params_t &p) {\n";
+        O << "  const int red_warps_ = " << red_warps(false) << "; (void)red_warps_;\n";
         O << "  extern __shared__ __align__(16) unsigned char op2g_smem[];\n";
         O << "  __shared__ __align__(8) unsigned long long bar_[3];\n";
         O << "  __shared__ int snu_[3][" << NSM << "];\n";
@@ -787,9 +791,38 @@ struct Gen {
         O << "    __syncthreads();\n";
         O << "    return;\n";
         O << "  }\n";
-        emit_global_reductions(true);
+        emit_global_reductions();
         O << "}\n\n";
         staging = false;
+    }
+
+    // Few packed components: the loop moves data rather than compute.
+    bool light_packs() const {
+        long long comps = 0;
+        for (size_t a = 0; a < S.args.size(); ++a) {
+            if (S.args[a].d.kind == OP2G_ARG_MAT) return false;
+            if (S.args[a].d.kind == OP2G_ARG_DAT) comps += dat_pack(a);
+        }
+        return comps <= 32;
+    }
+
+    // Increments of a column's layers.  On the usual extruded mesh the second
+    // half of a map's entries are the first half's one layer up (the top and
+    // the bottom nodes of a cell), so the top contributions of one layer and
+    // the bottom ones of the next, which the next lane holds, go to the same
+    // targets: they are added in registers and issued as one reduction, half
+    // as many for the L2, which is what bounds a light loop.  8.4 M prisms,
+    // six floats each: 44 -> PAIR_F32 us, doubles 81 -> PAIR_F64 us.  Whether
+    // the entries pair up is tested per column at run time.  Up to 12
+    // components: larger packs come with kernels that the FP64 pipe bounds,
+    // which the additions would only delay.
+    bool combines_layers(size_t a) const {
+        const op2g_arg_desc &d = S.args[a].d;
+        if (d.kind != OP2G_ARG_DAT || d.map < 0 || d.access != OP2G_INC || d.group != 0) return false;
+        const MapInfo &mi = S.maps[d.map];
+        return mi.kind == OP2G_MAP_PLAIN && nf == 1 && mi.arity % 2 == 0 &&
+               elt_size(d.dtype) == 8 && mi.arity * d.dim <= 12 && (int)mi.offset.size() == mi.arity &&
+               !S.loop.extruded_periodic && S.loop.scatter == OP2G_SCATTER_ATOMIC;
     }
 
     // A pure reduction: a flat loop over a whole set whose arguments are
@@ -847,13 +880,19 @@ struct Gen {
     // Few warps (small launches, and each work item of a batched launch, whose
     // loops have Globals of their own) go straight to the atomics, without the
     // barriers; so do loops of more than RED_MAX components (shared memory).
-    // Few means more for loops through maps, whose warps end far enough apart
-    // (320,000 triangles, action and area: 42 us either way at 10,000 warps
-    // with their own atomics, 43 with the barriers).
-    static constexpr int RED_MAX = 16, RED_WARPS = 2048, RED_WARPS_MAPS = 32768;
+    // Few means more for sweeping loops through maps, whose warps end far
+    // enough apart (320,000 triangles, action and area: 42 us at 10,000 warps
+    // with their own atomics, 43 with the barriers), and less for the balanced
+    // entry, whose warps end together (131,072 top cells, a sum of three
+    // floats in 4,256 warps: 15.7 -> 10.8 us).
+    static constexpr int RED_MAX = 16, RED_WARPS = 2048, RED_WARPS_MAPS = 32768,
+                         RED_WARPS_BALANCED = 1024;
 
-    // staged_run: a staged wrapper's own run function, launched alone.
-    void emit_global_reductions(bool staged_run = false) {
+    int red_warps(bool balanced) const {
+        return balanced ? RED_WARPS_BALANCED : S.maps.empty() ? RED_WARPS : RED_WARPS_MAPS;
+    }
+
+    void emit_global_reductions() {
         std::ostringstream &O = o;
         int comps = 0;
         for (const ArgInfo &A : S.args)
@@ -868,10 +907,17 @@ struct Gen {
         };
         const int W = S.block_size / 32;
         const bool cta = comps <= RED_MAX && W > 1;
+        // float sums always go through the CTA: each atomic rounds the running
+        // total, whatever the rest of the tree does (393,216 floats in 4,256
+        // warps: up to 6e-6 relative between two runs)
+        bool float_sum = false;
+        for (const ArgInfo &A : S.args)
+            float_sum = float_sum || (A.d.kind == OP2G_ARG_GLOBAL && A.d.access == OP2G_INC &&
+                                      A.d.dtype == OP2G_F32);
+        // (red_warps_: the entry point's threshold, negative for work items)
         if (cta)
-            O << "  const bool cta_ = " << (staged_run ? "" : "alone && ")
-              << "(long long)gridDim.x * (blockDim.x >> 5) > "
-              << (S.maps.empty() ? RED_WARPS : RED_WARPS_MAPS) << ";\n";
+            O << "  const bool cta_ = red_warps_ >= 0 && (long long)gridDim.x * (blockDim.x >> 5) > "
+              << (float_sum ? "1" : "red_warps_") << ";\n";
         for (size_t a = 0; a < S.args.size(); ++a) {
             const ArgInfo &A = S.args[a];
             if (A.d.kind != OP2G_ARG_GLOBAL || A.d.access == OP2G_READ) continue;
@@ -962,7 +1008,7 @@ struct Gen {
 
         // ----- the run function: a strided sweep of [start, end) plus reductions
         O << "__device__ __forceinline__ void op2g_run(const op2g_params_t &p, long long start, "
-             "long long end, long long first, long long stride, bool alone) {\n";
+             "long long end, long long first, long long stride, int red_warps_) {\n";
         emit_global_init();
         if (extr) {
             // pyop2/codegen/builder.py:771-812 (layer extents per iteration region)
@@ -1035,6 +1081,20 @@ struct Gen {
                             : 1;
         red_unroll = reduction_unroll();
         cells_per_thread = red_unroll ? red_unroll : cpt;
+        // A thread's (entity, layer) advances with its sweep instead of being
+        // divided out of the iteration number each time (a 64-bit division
+        // takes longer than all else in a light loop's iteration; most of it
+        // was hidden: 8.4 M prisms, a mean of six floats 37.7 -> 37 us).  Heavy
+        // kernels need the registers (prism elasticity VJP 2.24 against 2.26 ms).
+        const bool step_layers = extr && !varlay && cpt == 1 && light_packs();
+        layer_pairs = step_layers;
+        if (step_layers) {
+            O << "  const long long qs_ = nl_ ? op2g::div(stride, nl_) : 0;\n"
+              << "  const int rs_ = (int)(stride - qs_ * nl_);\n"
+              << "  const long long it0_ = i0_ + first + threadIdx.x;\n"
+              << "  long long it_ent = nl_ ? op2g::div(it0_, nl_) : 0;\n"
+              << "  int it_lay = (int)(it0_ - it_ent * nl_);\n";
+        }
         if (red_unroll) {
             O << "  for (long long base_ = i0_ + first; base_ < i1_; base_ += stride * " << red_unroll
               << ") {\n";
@@ -1093,12 +1153,23 @@ struct Gen {
                 }
             }
         }
+        for (size_t a = 0; layer_pairs && a < S.args.size(); ++a) {
+            if (!combines_layers(a)) continue;
+            const int ar = S.maps[S.args[a].d.map].arity;
+            O << I << ctype_of(S.args[a].d.dtype) << " t" << a << "[" << ar * S.args[a].d.dim << "];\n";
+            O << I << "int ti" << a << "[" << ar << "];\n";
+            O << I << "bool pr" << a << "_ = false;\n";
+        }
         O << I << (cpt > 1 ? "{\n" : "if (active) {\n");
         std::string J = "      ";
         // entity / layer
         if (extr && !varlay) {
-            O << J << "const long long it_ent = it / nl_;\n";
-            O << J << "const int layer = ls_ + (int)(it - it_ent * nl_);\n";
+            if (step_layers) {
+                O << J << "const int layer = ls_ + it_lay;\n";
+            } else {
+                O << J << "const long long it_ent = op2g::div(it, nl_);\n";
+                O << J << "const int layer = ls_ + (int)(it - it_ent * nl_);\n";
+            }
             O << J << "const long long n = " << (S.loop.indexed ? "p.indices[it_ent]" : "it_ent")
               << ";\n";
             O << J << "const int bottom = " << (S.loop.iteration_region == OP2G_ON_TOP ? "cs_" : "ls_")
@@ -1168,6 +1239,9 @@ struct Gen {
                 }
             }
         }
+        for (size_t a = 0; layer_pairs && a < S.args.size(); ++a)
+            if (combines_layers(a)) emit_layer_pairs(a, I);
+        layer_pairs = false;
         if (any_shared) {
             // The sweep step is uniform across the CTA (base_ depends on the
             // block only), so these barriers are reached by every thread.
@@ -1189,6 +1263,9 @@ struct Gen {
             O << "    __syncthreads();\n";
             O << "    par_ ^= 1;\n";
         }
+        if (step_layers)
+            O << "    it_ent += qs_;\n    it_lay += rs_;\n"
+              << "    if (it_lay >= nl_) { it_lay -= (int)nl_; ++it_ent; }\n";
         if (cpt > 1 || red_unroll) O << "   }\n";  // cells of the step
         O << "  }\n";  // sweep loop
         guard_unpack = false;
@@ -1209,7 +1286,7 @@ struct Gen {
             O << "extern \"C\" __global__ void __launch_bounds__(" << BS
               << ") op2g_wrap(const __grid_constant__ op2g_params_t p) {\n"
               << "  op2g_run(p, p.start, p.end, (long long)blockIdx.x * " << bdim
-              << ", (long long)gridDim.x * " << bdim << ", true);\n}\n";
+              << ", (long long)gridDim.x * " << bdim << ", " << red_warps(false) << ");\n}\n";
         }
         if (!any_shared && !any_staged) {
             // Balanced form for launches of a few CTAs per SM: CTA b takes the
@@ -1221,14 +1298,15 @@ struct Gen {
               << "  const long long c_ = (n_ + gridDim.x - 1) / gridDim.x;\n"
               << "  const long long s_ = p.start + (long long)blockIdx.x * c_;\n"
               << "  const long long e_ = s_ + c_ < p.end ? s_ + c_ : p.end;\n"
-              << "  if (s_ < e_) op2g_run(p, s_, e_, 0, (long long)blockDim.x, true);\n}\n";
+              << "  if (s_ < e_) op2g_run(p, s_, e_, 0, (long long)blockDim.x, "
+              << red_warps(true) << ");\n}\n";
         }
         O << "extern \"C\" __global__ void __launch_bounds__(" << BS
           << ") op2g_wrap_batched(const op2g_params_t *__restrict__ P, const long long "
              "*__restrict__ work, long long nwork) {\n"
           << "  for (long long w = blockIdx.x; w < nwork; w += gridDim.x) {\n"
           << "    const op2g_params_t &p = P[work[3 * w]];\n"
-          << "    op2g_run(p, work[3 * w + 1], work[3 * w + 2], 0, " << BS << ", false);\n"
+          << "    op2g_run(p, work[3 * w + 1], work[3 * w + 2], 0, " << BS << ", -1);\n"
           << "  }\n}\n";
         return O.str();
     }
@@ -1255,6 +1333,56 @@ struct Gen {
         }
     }
 
+    // Scatter of a combines_layers argument, by all lanes of the warp (whose
+    // iterations are consecutive: lane - 1 holds the layer below, unless this
+    // is the column's first).
+    void emit_layer_pairs(size_t a, const std::string &I) {
+        std::ostringstream &O = o;
+        const ArgInfo &A = S.args[a];
+        const char *T = ctype_of(A.d.dtype);
+        const int ar = S.maps[A.d.map].arity, D = A.d.dim, h = ar / 2;
+        const std::string an = std::to_string(a);
+        O << I << "{ " << T << " *d_ = (" << T << " *)p.ptr[" << A.slot << "];\n";
+        O << I << "  const int lane_ = threadIdx.x & 31;\n";
+        O << I << "  const bool tx_ = pr" << an << "_ && lane_ < 31 && it_lay + 1 < nl_ && it + 1 < i1_;\n";
+        O << I << "  if (__any_sync(0xffffffffu, pr" << an << "_)) {\n";
+        O << I << "    const bool rx_ = pr" << an << "_ && lane_ > 0 && it_lay > 0;\n";
+        O << "#pragma unroll\n" << I << "    for (int k = 0; k < " << h * D << "; ++k) {\n";
+        O << I << "      const " << T << " v_ = __shfl_up_sync(0xffffffffu, t" << an << "[k + " << h * D
+          << "], 1);\n";
+        O << I << "      if (rx_) t" << an << "[k] += v_;\n";
+        O << I << "    }\n" << I << "  }\n";
+        O << I << "  if (active) {\n";
+        O << "#pragma unroll\n" << I << "    for (int i = 0; i < " << ar << "; ++i) {\n";
+        O << I << "      if (ti" << an << "[i] < 0 || (i >= " << h << " && tx_)) continue;\n";
+        O << "#pragma unroll\n" << I << "      for (int j = 0; j < " << D << "; ++j) op2g::atomic_inc(&d_[(long long)ti"
+          << an << "[i] * " << gstride(a) << " + j], t" << an << "[i * " << D << " + j]);\n";
+        O << I << "    }\n" << I << "  }\n" << I << "}\n";
+    }
+
+    // READ / RW / MIN / MAX pack of an indirect Dat argument; `checked`: map
+    // entries may be negative (their components are 0).
+    void emit_gather(size_t a, const std::string &J, bool checked) {
+        std::ostringstream &O = o;
+        const ArgInfo &A = S.args[a];
+        const char *T = ctype_of(A.d.dtype);
+        const int ar = S.maps[A.d.map].arity, D = A.d.dim;
+        const bool nc = S.loop.nc_reads && A.d.access == OP2G_READ;
+        O << J << "{ const " << T << " *d_ = (const " << T << " *)p.ptr[" << A.slot << "];\n";
+        for (int f = 0; f < nf; ++f) {
+            O << J << "#pragma unroll\n";
+            O << J << "  for (int i = 0; i < " << ar << "; ++i) {\n";
+            O << J << "    const int x_ = " << idx_arr(A.d.map, f) << "[i];\n";
+            O << J << "#pragma unroll\n";
+            O << J << "    for (int j = 0; j < " << D << "; ++j) t" << first[a] << "[" << poff[a]
+              << " + (" << f * ar << " + i) * " << D << " + j] = " << (checked ? "x_ >= 0 ? " : "")
+              << (nc ? "__ldg(&" : "") << "d_[(long long)x_ * " << gstride(a) << " + j]"
+              << (nc ? ")" : "") << (checked ? std::string(" : (") + T + ")0" : "") << ";\n";
+            O << J << "  }\n";
+        }
+        O << J << "}\n";
+    }
+
     // Pack, call, unpack for one iteration (entity n, and layer when extruded).
     void emit_body(const std::string &J, bool warp, bool plain, bool rows_prefetched = false) {
         std::ostringstream &O = o;
@@ -1276,6 +1404,26 @@ struct Gen {
         }
         for (size_t m = 0; m < S.maps.size(); ++m)
             if (used[m]) emit_index_arrays((int)m, J);
+
+        // Whether all of the iteration's map entries are non-negative (they are
+        // on any ordinary mesh): in light extruded loops one test instead of
+        // one per entry and access.  8.4 M prisms, a mean of six floats: 111 ->
+        // 93 warp instructions per 32 cells, 37 -> 32 us.  Flat loops of the
+        // same kind wait for their gathers and gain nothing; large packs lose
+        // (the code doubles: prism elasticity VJP 2.24 -> 2.27 ms).
+        const bool one_test = S.loop.extruded && !staging && light_packs();
+        std::vector<size_t> gathers;   // indirect Dats read through global memory
+        std::string all_ok;
+        for (size_t m = 0; one_test && m < S.maps.size(); ++m) {
+            if (!used[m]) continue;
+            std::string any;
+            for (int f = 0; f < nf; ++f)
+                for (int i = 0; i < S.maps[m].arity; ++i)
+                    any += (any.empty() ? "" : " | ") + idx_arr((int)m, f) + "[" + std::to_string(i) + "]";
+            O << J << "const int any" << m << "_ = " << any << ";\n";
+            all_ok += (all_ok.empty() ? "" : " | ") + ("any" + std::to_string(m) + "_");
+        }
+        if (!all_ok.empty()) O << J << "const bool all_ok_ = (" << all_ok << ") >= 0;\n";
 
         // Packs (pyop2/codegen/builder.py:240-300, 303-365, 531-552)
         std::vector<std::string> kargs;
@@ -1332,7 +1480,8 @@ struct Gen {
                 const int tot = psize[first[a]];
                 const std::string tn = "t" + std::to_string(first[a]);
                 const std::string po = std::to_string(poff[a]) + " + ";
-                const bool decl_outside = warp && A.d.access == OP2G_INC;
+                const bool decl_outside = (warp && A.d.access == OP2G_INC) ||
+                                          (layer_pairs && combines_layers(a));
                 if (lead && !decl_outside) O << J << T << " " << tn << "[" << tot << "];\n";
                 if (A.d.access == OP2G_INC || A.d.access == OP2G_WRITE) {
                     if (lead) {
@@ -1354,21 +1503,7 @@ struct Gen {
                       << " + j] : (" << T << ")0;\n";
                     O << J << "}\n";
                 } else {
-                    O << J << "{ const " << T << " *d_ = (const " << T << " *)p.ptr[" << A.slot
-                      << "];\n";
-                    for (int f = 0; f < nf; ++f) {
-                        O << J << "#pragma unroll\n";
-                        O << J << "  for (int i = 0; i < " << ar << "; ++i) {\n";
-                        O << J << "    const int x_ = " << idx_arr(A.d.map, f) << "[i];\n";
-                        O << J << "#pragma unroll\n";
-                        const bool nc = S.loop.nc_reads && A.d.access == OP2G_READ;
-                        O << J << "    for (int j = 0; j < " << D << "; ++j) " << tn << "[" << po
-                          << "(" << f * ar << " + i) * " << D << " + j] = x_ >= 0 ? "
-                          << (nc ? "__ldg(&" : "") << "d_[(long long)x_ * " << gstride(a) << " + j]"
-                          << (nc ? ")" : "") << " : (" << T << ")0;\n";
-                        O << J << "  }\n";
-                    }
-                    O << J << "}\n";
+                    gathers.push_back(a);
                 }
                 if (lead) kargs.push_back("op2g::ptr(" + tn + ")");
             } else if (A.d.kind == OP2G_ARG_MAT) {
@@ -1381,6 +1516,15 @@ struct Gen {
                   << ";\n";
                 kargs.push_back("op2g::ptr(t" + an + ")");
             }
+        }
+        if (one_test && !gathers.empty()) {
+            O << J << "if (all_ok_) {\n";
+            for (size_t a : gathers) emit_gather(a, J + "  ", false);
+            O << J << "} else {\n";
+            for (size_t a : gathers) emit_gather(a, J + "  ", true);
+            O << J << "}\n";
+        } else {
+            for (size_t a : gathers) emit_gather(a, J, true);
         }
         if (S.loop.pass_layer_arg) kargs.push_back("layer");
         if (declared_without_parameters(S.user_src, S.kernel_name)) kargs.clear();
@@ -1414,6 +1558,19 @@ struct Gen {
                           << " + i] = " << idx_arr(A.d.map, f) << "[i];\n";
                     continue;  // scattered after the active block
                 }
+                if (layer_pairs && combines_layers(a)) {   // scattered after the active block
+                    const int h = ar / 2;
+                    const std::string mi = idx_arr(A.d.map, 0);
+                    O << J << "#pragma unroll\n" << J << "for (int i = 0; i < " << ar << "; ++i) ti" << an
+                      << "[i] = " << mi << "[i];\n";
+                    O << J << "pr" << an << "_ = ti" << an << "[0] >= 0";
+                    for (int i = 1; i < h; ++i) O << " && ti" << an << "[" << i << "] >= 0";
+                    for (int i = 0; i < h; ++i)
+                        O << " && " << mi << "[" << i + h << "] == " << mi << "[" << i << "] + "
+                          << S.maps[A.d.map].offset[i];
+                    O << ";\n";
+                    continue;
+                }
                 if (staging && st_arg[a] >= 0) {
                     // staged INC: each entry owns its slot (plain store); the
                     // slots of one target are summed when the partition is done
@@ -1427,12 +1584,14 @@ struct Gen {
                     O << J << "}\n";
                     continue;
                 }
+                for (int checked = one_test ? 0 : 1; checked < 2; ++checked) {
+                if (one_test) O << J << (checked ? "else " : "if (all_ok_) ");
                 O << J << "{ " << T << " *d_ = (" << T << " *)p.ptr[" << A.slot << "];\n";
                 for (int f = 0; f < nf; ++f) {
                     O << J << "#pragma unroll\n";
                     O << J << "  for (int i = 0; i < " << ar << "; ++i) {\n";
                     O << J << "    const int x_ = " << idx_arr(A.d.map, f) << "[i];\n";
-                    O << J << "    if (x_ < 0) continue;\n";
+                    if (checked) O << J << "    if (x_ < 0) continue;\n";
                     if (shared_ts[a]) {
                         // find or claim x_'s slot (bounded linear probing;
                         // a full table sends the contribution to global memory)
@@ -1478,6 +1637,7 @@ struct Gen {
                     O << J << "  }\n";
                 }
                 O << J << "}\n";
+                }
             } else if (A.d.kind == OP2G_ARG_MAT) {
                 // MatSetValuesBlockedLocal(ADD|INSERT) on block-CSR storage.
                 const int ra = S.maps[A.d.map].arity, ca = S.maps[A.d.cmap].arity;

@@ -60,6 +60,11 @@ struct anyptr {
 template <class T>
 __device__ __forceinline__ anyptr<T> ptr(T *p) { return anyptr<T>(p); }
 
+// a / b for a >= 0, b > 0, in 32 bits where they fit.
+__device__ __forceinline__ long long div(long long a, long long b) {
+    return ((a | b) >> 32) ? a / b : (long long)((unsigned)a / (unsigned)b);
+}
+
 __device__ __forceinline__ void set_err(int *err, int bit) {
     if (err) atomicOr(err, bit);
 }
