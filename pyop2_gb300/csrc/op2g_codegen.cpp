@@ -92,6 +92,64 @@ static bool declared_without_parameters(const std::string &src, const std::strin
     return false;
 }
 
+// True when the user kernel plainly does next to no arithmetic: its body has
+// no multiplication, division or remainder, calls nothing, and adds or
+// subtracts in at most eight places, in loops that are not nested (a scatter
+// of cell values, a valence count).  Anything it cannot see through is "no".
+static bool moves_data(const std::string &src, const std::string &name) {
+    std::string t;   // without comments
+    for (size_t i = 0; i < src.size(); ++i) {
+        if (src.compare(i, 2, "/*") == 0) {
+            const size_t e = src.find("*/", i + 2);
+            if (e == std::string::npos) return false;
+            i = e + 1;
+            t += ' ';
+        } else if (src.compare(i, 2, "//") == 0) {
+            const size_t e = src.find('\n', i);
+            if (e == std::string::npos) break;
+            i = e;
+            t += ' ';
+        } else {
+            t += src[i];
+        }
+    }
+    auto ident = [](char c) { return std::isalnum((unsigned char)c) || c == '_'; };
+    if (t.find('#') != std::string::npos || t.find('"') != std::string::npos) return false;
+    // one function only: name ( parameters ) { body }
+    size_t p = t.find(name);
+    while (p != std::string::npos && ((p > 0 && ident(t[p - 1])) || ident(t[p + name.size()])))
+        p = t.find(name, p + 1);
+    if (p == std::string::npos) return false;
+    const size_t open = t.find('{', p), paren = t.find(')', p);
+    if (open == std::string::npos || paren == std::string::npos || paren > open ||
+        t.find('{') != open)
+        return false;
+    const std::string body = t.substr(open);
+    int adds = 0, loops = 0;
+    for (size_t i = 0; i < body.size(); ++i) {
+        const char c = body[i];
+        if (c == '*' || c == '/' || c == '%') return false;
+        if (c == '+' || c == '-') {
+            ++adds;
+            if (i + 1 < body.size() && body[i + 1] == c) {   // ++ and -- of a loop
+                --adds;
+                ++i;
+            }
+        }
+        if (!ident(c)) continue;
+        size_t e = i;
+        while (e < body.size() && ident(body[e])) ++e;
+        const std::string word = body.substr(i, e - i);
+        size_t q = e;
+        while (q < body.size() && std::isspace((unsigned char)body[q])) ++q;
+        if (word == "while" || word == "do" || word == "goto") return false;
+        if (word == "for") ++loops;
+        if (q < body.size() && body[q] == '(' && word != "for" && word != "if") return false;
+        i = e - 1;
+    }
+    return adds <= 8 && loops <= 2;
+}
+
 // Starting value of an INC accumulator (Global, Dat and Mat packs; the
 // reference zero-fills them, pyop2/codegen/builder.py:271-274, 353-356,
 // 538-541).  For floating types it is -0.0, the exact identity of IEEE
@@ -232,6 +290,7 @@ struct Gen {
     // Arguments whose INC contributions neighbouring layers combine
     // (combines_layers); set while a run function that does so is written.
     bool layer_pairs = false;
+    bool cell_pairs = false;   // the same for neighbouring cells (combines_cells)
 
     explicit Gen(const Signature &s) : S(s) {
         nf = (S.loop.extruded && S.loop.iteration_region == OP2G_ON_INTERIOR_FACETS) ? 2 : 1;
@@ -825,6 +884,54 @@ struct Gen {
                !S.loop.extruded_periodic && S.loop.scatter == OP2G_SCATTER_ATOMIC;
     }
 
+    // Increments of neighbouring cells.  Consecutive cells of a mesh share
+    // most of their targets, and the L2 takes each lane's reduction of a
+    // shared target by itself: that rate bounds a loop that does little else.
+    // Lanes 2k and 2k + 1 therefore add what they have for a common target in
+    // registers and issue it once; then lanes 4k and 4k + 2.  12.6 M tets, four
+    // entries each, lexicographic / random numbering: floats 99 / 245 -> 75 /
+    // 143 us, doubles 119 / 250 -> 92 / 172 us.
+    // The additions are free for 4-byte and integer types.  Doubles pay for
+    // them on the FP64 pipe (2 per clock per SM): one round only (two: 161 /
+    // 165 us), and only in kernels that leave the pipe idle (moves_data); the
+    // P1 Laplacian action, 63 FP64 instructions per cell, would lose 5 %.
+    bool combines_cells(size_t a) const {
+        const op2g_arg_desc &d = S.args[a].d;
+        if (S.loop.extruded || S.loop.scatter != OP2G_SCATTER_ATOMIC || any_staged) return false;
+        if (d.kind != OP2G_ARG_DAT || d.map < 0 || d.access != OP2G_INC || d.group != 0) return false;
+        return S.maps[d.map].arity * d.dim <= 16 &&
+               (d.dtype != OP2G_F64 || moves_data(S.user_src, S.kernel_name));
+    }
+
+    // Scatter of a combines_cells argument, by all lanes of the warp.
+    void emit_cell_pairs(size_t a, const std::string &I) {
+        std::ostringstream &O = o;
+        const ArgInfo &A = S.args[a];
+        const char *T = ctype_of(A.d.dtype);
+        const int ar = S.maps[A.d.map].arity, D = A.d.dim;
+        const std::string an = std::to_string(a);
+        O << I << "{ " << T << " *d_ = (" << T << " *)p.ptr[" << A.slot << "];\n";
+        O << "#pragma unroll\n" << I << "  for (int i = 0; i < " << ar << "; ++i) {\n";
+        O << I << "    int x_ = active ? ti" << an << "[i] : -1;\n";   // -1: nothing (left) to add
+        for (int step = 1; step <= (A.d.dtype == OP2G_F64 ? 1 : 2); step *= 2) {
+            // every lane takes part in the shuffles, whatever it holds
+            O << I << "    { const int o_ = __shfl_xor_sync(0xffffffffu, x_, " << step << ");\n";
+            O << I << "      const bool same_ = x_ >= 0 && o_ == x_;\n";
+            O << I << "      if (__any_sync(0xffffffffu, same_)) {\n";
+            O << "#pragma unroll\n" << I << "        for (int j = 0; j < " << D << "; ++j) {\n";
+            O << I << "          const " << T << " v_ = __shfl_xor_sync(0xffffffffu, t" << an << "[i * "
+              << D << " + j], " << step << ");\n";
+            O << I << "          if (same_) t" << an << "[i * " << D << " + j] += v_;\n";
+            O << I << "        }\n" << I << "      }\n";
+            O << I << "      if (same_ && (threadIdx.x & " << step << ")) x_ = -1; }\n";
+        }
+        O << I << "    if (x_ < 0) continue;\n";
+        O << "#pragma unroll\n" << I << "    for (int j = 0; j < " << D
+          << "; ++j) op2g::atomic_inc(&d_[(long long)x_ * " << gstride(a) << " + j], t" << an << "[i * "
+          << D << " + j]);\n";
+        O << I << "  } }\n";
+    }
+
     // A pure reduction: a flat loop over a whole set whose arguments are
     // Globals and direct READ Dats of a few bytes per entity.  Its threads
     // load the rows of several iterations (up to 64 bytes) before the first
@@ -1088,6 +1195,7 @@ struct Gen {
         // kernels need the registers (prism elasticity VJP 2.24 against 2.26 ms).
         const bool step_layers = extr && !varlay && cpt == 1 && light_packs();
         layer_pairs = step_layers;
+        cell_pairs = !extr && cpt == 1;
         if (step_layers) {
             O << "  const long long qs_ = nl_ ? op2g::div(stride, nl_) : 0;\n"
               << "  const int rs_ = (int)(stride - qs_ * nl_);\n"
@@ -1153,12 +1261,12 @@ struct Gen {
                 }
             }
         }
-        for (size_t a = 0; layer_pairs && a < S.args.size(); ++a) {
-            if (!combines_layers(a)) continue;
+        for (size_t a = 0; a < S.args.size(); ++a) {
+            if (!deferred(a)) continue;
             const int ar = S.maps[S.args[a].d.map].arity;
             O << I << ctype_of(S.args[a].d.dtype) << " t" << a << "[" << ar * S.args[a].d.dim << "];\n";
             O << I << "int ti" << a << "[" << ar << "];\n";
-            O << I << "bool pr" << a << "_ = false;\n";
+            if (layer_pairs) O << I << "bool pr" << a << "_ = false;\n";
         }
         O << I << (cpt > 1 ? "{\n" : "if (active) {\n");
         std::string J = "      ";
@@ -1239,9 +1347,9 @@ struct Gen {
                 }
             }
         }
-        for (size_t a = 0; layer_pairs && a < S.args.size(); ++a)
-            if (combines_layers(a)) emit_layer_pairs(a, I);
-        layer_pairs = false;
+        for (size_t a = 0; a < S.args.size(); ++a)
+            if (deferred(a)) layer_pairs ? emit_layer_pairs(a, I) : emit_cell_pairs(a, I);
+        layer_pairs = cell_pairs = false;
         if (any_shared) {
             // The sweep step is uniform across the CTA (base_ depends on the
             // block only), so these barriers are reached by every thread.
@@ -1331,6 +1439,11 @@ struct Gen {
             default:
                 o << ind << "const int " << ls << " = " << cs << ", " << le << " = " << ce << ";\n";
         }
+    }
+
+    // Scattered by the whole warp after the active block.
+    bool deferred(size_t a) const {
+        return (layer_pairs && combines_layers(a)) || (cell_pairs && combines_cells(a));
     }
 
     // Scatter of a combines_layers argument, by all lanes of the warp (whose
@@ -1481,7 +1594,7 @@ struct Gen {
                 const std::string tn = "t" + std::to_string(first[a]);
                 const std::string po = std::to_string(poff[a]) + " + ";
                 const bool decl_outside = (warp && A.d.access == OP2G_INC) ||
-                                          (layer_pairs && combines_layers(a));
+                                          deferred(a);
                 if (lead && !decl_outside) O << J << T << " " << tn << "[" << tot << "];\n";
                 if (A.d.access == OP2G_INC || A.d.access == OP2G_WRITE) {
                     if (lead) {
@@ -1558,11 +1671,12 @@ struct Gen {
                           << " + i] = " << idx_arr(A.d.map, f) << "[i];\n";
                     continue;  // scattered after the active block
                 }
-                if (layer_pairs && combines_layers(a)) {   // scattered after the active block
+                if (deferred(a)) {   // scattered after the active block
                     const int h = ar / 2;
                     const std::string mi = idx_arr(A.d.map, 0);
                     O << J << "#pragma unroll\n" << J << "for (int i = 0; i < " << ar << "; ++i) ti" << an
                       << "[i] = " << mi << "[i];\n";
+                    if (!layer_pairs) continue;
                     O << J << "pr" << an << "_ = ti" << an << "[0] >= 0";
                     for (int i = 1; i < h; ++i) O << " && ti" << an << "[" << i << "] >= 0";
                     for (int i = 0; i < h; ++i)
