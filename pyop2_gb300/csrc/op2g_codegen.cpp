@@ -1380,6 +1380,22 @@ struct Gen {
         emit_global_reductions();
         O << "}\n\n";
 
+        // Wrappers whose element matrix does not fit in registers keep it (and
+        // what the kernel computes it from) in local memory however many
+        // registers they get; more resident threads then hide its latency
+        // better than the registers do.  18 x 18 prism elasticity matrices,
+        // 262,144 prisms: 254 registers 4.05 ms, 128 3.13, 96 3.05, 80 3.02,
+        // 64 3.03, 48 3.08, 40 3.26; 768 threads per SM ask for 80.  Launches of
+        // the balanced entry are too short for that (1,000 prisms 0.29 against
+        // 0.32 ms), and it keeps the registers.
+        bool local_matrix = false;
+        for (size_t a = 0; a < S.args.size(); ++a)
+            local_matrix = local_matrix || (S.args[a].d.kind == OP2G_ARG_MAT && first[a] == (int)a &&
+                                            psize[a] >= 128);
+        const std::string bounds =
+            std::to_string(BS) +
+            (local_matrix && BS <= 384 ? ", " + std::to_string(768 / BS) : std::string());
+
         // ----- the entry points.  Without shared-memory staging (whose
         // tables are sized for BS threads) the wrapper may be launched with
         // fewer threads per CTA than BS: a small iteration set is then
@@ -1391,7 +1407,7 @@ struct Gen {
               << ") op2g_wrap(const __grid_constant__ op2g_params_t p) {\n"
               << "  op2g_run_staged(p);\n}\n";
         } else {
-            O << "extern \"C\" __global__ void __launch_bounds__(" << BS
+            O << "extern \"C\" __global__ void __launch_bounds__(" << bounds
               << ") op2g_wrap(const __grid_constant__ op2g_params_t p) {\n"
               << "  op2g_run(p, p.start, p.end, (long long)blockIdx.x * " << bdim
               << ", (long long)gridDim.x * " << bdim << ", " << red_warps(false) << ");\n}\n";

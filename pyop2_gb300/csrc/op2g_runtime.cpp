@@ -218,6 +218,7 @@ struct Loaded {
     int regs = -1;
     int occ = 0;  // resident CTAs per SM
     int occ_small = 0;  // the same for CTAs of SMALL_CTA threads
+    int occ_chunked = 0;  // resident CTAs per SM of the balanced entry
     int sms = 0;
     // staged wrappers: dynamic shared memory the function is set up for, and
     // the resident CTAs per SM at the last size asked for
@@ -256,6 +257,9 @@ op2g_status load_module(const std::string &cubin, const char *fname, const char 
     D.FuncGetAttribute(&L.regs, CU_FUNC_ATTRIBUTE_NUM_REGS, L.f);
     if (D.OccupancyMaxActiveBlocksPerMultiprocessor(&L.occ, L.f, bs, 0) != CUDA_SUCCESS) L.occ = 1;
     if (L.occ < 1) L.occ = 1;
+    if (!L.fc || D.OccupancyMaxActiveBlocksPerMultiprocessor(&L.occ_chunked, L.fc, bs, 0) !=
+                     CUDA_SUCCESS)
+        L.occ_chunked = L.occ;
     if (bs > SMALL_CTA && D.OccupancyMaxActiveBlocksPerMultiprocessor(
                               &L.occ_small, L.f, SMALL_CTA, 0) != CUDA_SUCCESS)
         L.occ_small = 0;
@@ -344,7 +348,7 @@ static void refine_shape(const Loaded &L, const Signature &S, int64_t items, int
     // as long as an iteration alone (79,380 prisms on 77,824 resident threads,
     // action: 0.492 against 0.536 ms; assembly gains all the same, 1.60 -> 1.30).
     const int64_t round = (int64_t)L.occ_small * SMALL_CTA * L.sms;
-    if (*chunked && (*grid <= (int64_t)L.occ * L.sms ||
+    if (*chunked && (*grid <= (int64_t)L.occ_chunked * L.sms ||
                      (!mat && items > round && items < round + round / 7)))
         return;
     if (!use) {
