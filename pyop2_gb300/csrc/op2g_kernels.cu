@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(256)
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int ra = P.rarity, tr = P.tr;
+    const bool vec4 = ra % 4 == 0 && (unsigned long long)P.rmap % 16 == 0;
     const long long nvirt = P.nvirt, stride = (long long)gridDim.x * blockDim.x;
     for (long long v0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); v0 < nvirt;
          v0 += stride) {   // v0 is the same for a warp's lanes
@@ -147,6 +148,14 @@ __global__ void __launch_bounds__(256)
         for (int i0 = 0; i0 < tr; i0 += 4) {
             int r[4], head[4], n[4];
             long long at[4];
+            if (EMODE == E_FLAT && vec4) {   // flat rows of whole, aligned int4
+                int4 t = make_int4(-1, -1, -1, -1);
+                if (ok) t = __ldg((const int4 *)(P.rmap + v * ra + i0));
+                r[0] = t.x;
+                r[1] = t.y;
+                r[2] = t.z;
+                r[3] = t.w;
+            } else
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int i = i0 + q, k = i >= ra;
@@ -408,8 +417,8 @@ __device__ __forceinline__ void sort_network(unsigned (&v)[N]) {
 // so no two lanes conflict), sorts the distinct ones in registers, and the
 // warp stores the rows packed.  There are no ballots, barriers or shuffles per
 // row: 197 warp instructions per row of the tet mesh against 306 for the
-// warp-per-row form, 0.29 against 0.39 ms at 6 M cells (bound by issue slots
-// and the latency of the lists and map rows; tables of 40-64 places take fewer
+// warp-per-row form, 0.29 (0.24 with the loads one entry ahead) against 0.39 ms
+// at 6 M cells (bound by issue slots; tables of 40-64 places take fewer
 // probes but leave fewer warps resident: 0.28-0.35 ms; entering four columns
 // together, a probe of each lane at a time, 0.34 ms).  A batch with a row of
 // more than THREAD_MAX distinct columns returns -1 and runs the other form.
@@ -460,6 +469,21 @@ __device__ __forceinline__ int rows_by_lane(const SpDev &S, const PairDev *__res
             }
         }
     };
+    if (EMODE == E_FLAT && A.vec4 && A.ca == 4) {
+        // the commonest rows: the next entry's columns are on their way while
+        // the current ones are entered (6 M cells 0.29 -> 0.24 ms; the same for
+        // every kind of entry, in one loop, took 0.27)
+        const int *ents = (const int *)list;
+        const int4 *rows = (const int4 *)A.cmap;
+        int4 next = m > 0 ? __ldg(rows + __ldg(ents)) : make_int4(-1, -1, -1, -1);
+        int ent = m > 1 ? __ldg(ents + 1) : 0;
+        for (int e = 0; e < m && !over; ++e) {
+            int c[4] = {next.x, next.y, next.z, next.w};
+            if (e + 1 < m) next = __ldg(rows + ent);
+            if (e + 2 < m) ent = __ldg(ents + e + 2);
+            enter(c);
+        }
+    } else
     for (int e = 0; e < m && !over; ++e) {
         const int *row = nullptr, *coff = nullptr, *cq = nullptr;
         int layer = 0;
