@@ -1272,6 +1272,21 @@ struct Gen {
         std::string J = "      ";
         // entity / layer
         if (extr && !varlay) {
+            // Map rows of the next iteration's column, another one, are brought
+            // to the L2 (a hint; nothing it reads is used): the row is the first
+            // of two loads that wait for each other.  8.4 M prisms out of
+            // memory, a mean of six floats: 47 -> 39 us.  Loops that combine
+            // their increments wait for the FP64 pipe instead and lose 3 %.
+            bool combined = false;
+            for (size_t a = 0; a < S.args.size(); ++a) combined = combined || deferred(a);
+            if (step_layers && !S.loop.indexed && !combined) {
+                O << J << "if (it + stride < i1_) {\n";
+                for (size_t m = 0; m < S.maps.size(); ++m)
+                    if (rows[m])
+                        O << J << "  asm volatile(\"prefetch.global.L2 [%0];\" :: \"l\"((const int *)p.ptr["
+                          << S.map_slot((int)m) << "] + (it_ent + qs_) * " << S.maps[m].arity << "));\n";
+                O << J << "}\n";
+            }
             if (step_layers) {
                 O << J << "const int layer = ls_ + it_lay;\n";
             } else {
