@@ -385,6 +385,10 @@ op2g_status op2g_mat_set_diagonal(const op2g_bcsr *m, const int32_t *rows_dev, i
 /* y = A x (transpose = 0) or y = A^T x (transpose = 1; y must be zeroed, uses atomics). */
 op2g_status op2g_mat_spmv(const op2g_bcsr *m, const double *x, double *y, int32_t transpose,
                           void *stream);
+/* The same for a caller that knows the number of stored blocks (-1: unknown),
+ * which lets large CSR matrices (1 x 1 blocks) stream through bulk copies. */
+op2g_status op2g_mat_spmv_sized(const op2g_bcsr *m, int64_t nblocks, const double *x, double *y,
+                                int32_t transpose, void *stream);
 
 /* ------------------------------------------------------------ colouring */
 /* Greedy colouring of `ncells` entities so that no two entities of one colour

@@ -114,6 +114,7 @@ SIGNATURES = {
     "op2g_mat_zero_rows": (_i32, [ctypes.POINTER(BCSR), _p, _i64, ctypes.c_double, _p]),
     "op2g_mat_set_diagonal": (_i32, [ctypes.POINTER(BCSR), _p, _i64, ctypes.c_double, _p, _p]),
     "op2g_mat_spmv": (_i32, [ctypes.POINTER(BCSR), _p, _p, _i32, _p]),
+    "op2g_mat_spmv_sized": (_i32, [ctypes.POINTER(BCSR), _i64, _p, _p, _i32, _p]),
     "op2g_colour_workspace": (_i32, [_i64, _i32, ctypes.POINTER(_i64),
                                      ctypes.POINTER(ctypes.c_size_t)]),
     "op2g_colour": (_i32, [_i64, _i32, ctypes.POINTER(_p), _pi32, ctypes.POINTER(_i64), _i32,

@@ -1686,6 +1686,164 @@ cudaError_t spmv_lane_launch(cudaStream_t st, const op2g_bcsr &m, const double *
     return spmv_lane_go<R, C, K, MINB, 1, TR>(st, m, x, y);
 }
 
+// ---- CSR through bulk copies
+//
+// The lane kernel above reads each lane's own row, so a load instruction
+// touches 32 rows' lines.  Here a warp's 32 rows, which are one contiguous run
+// of entries, arrive in its shared memory by two bulk copies (values, columns),
+// and the lanes read them from there (rows of 15 entries: next to no bank
+// conflicts); only the x values go through the L1.  What bounds it is the
+// latency of a batch (copies, then x, then the FP64 chain of a row), so many
+// warps with one small buffer each beat fewer with two: 128^3 tet mesh, 31.8 M
+// entries, by warps per SM (one buffer of 512 entries) 14: 105 us, 18: 91,
+// 22: 85, 26: 81.6; two buffers, 18 warps: 84; the lane kernel 89.7.  But the
+// misses of x need room in the L1: the buffers are held to about three
+// quarters of it (36 warps: 76 us with lexicographic, 229 with random vertex
+// numbering; 26 warps: 140 with random numbering, the lane kernel 173).
+// Transposed 95 -> 87 us.  The sums run in the lane kernel's order, so the
+// results are its bit for bit.
+//
+// A batch that does not fit the buffer, or whose copies (rounded to 16 bytes)
+// would end past the arrays, is read from global memory.  Every wait is
+// bounded: when one gives up, the warp reads that batch and all later ones
+// from global memory, and waits (bounded) for its copies before it ends.
+__device__ __forceinline__ unsigned smem_u32(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned bytes,
+                                          unsigned long long *bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+            smem_u32(dst)),
+        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity) {
+    for (int it = 0; it < (1 << 20); ++it) {
+        unsigned done;
+        asm volatile(
+            "{\n .reg .pred p_;\n mbarrier.try_wait.parity.shared::cta.b64 p_, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p_;\n}" : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+
+constexpr int BULK_WARPS = 2, BULK_SMEM_PER_SM = 163 * 1024, BULK_CARVEOUT = 75;
+
+template <bool TR>
+__global__ void __launch_bounds__(32 * BULK_WARPS)
+    k_spmv_csr_bulk(op2g_bcsr m, long long nnz, int cap, const double *__restrict__ x,
+                    double *__restrict__ y) {
+    extern __shared__ __align__(16) unsigned char bulk_smem[];
+    __shared__ __align__(8) unsigned long long bars[BULK_WARPS];
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long *bar = &bars[warp];
+    double *sv = (double *)(bulk_smem + (size_t)warp * cap * 12);
+    int *sc = (int *)(sv + cap);
+    if (lane == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncwarp();
+    const long long nb = (m.nrows + 31) / 32, step = (long long)gridDim.x * BULK_WARPS;
+    bool alive = true;       // no wait has given up
+    unsigned phase = 0;
+    // row bounds of this lane in batch b (empty past the last row)
+    auto bounds = [&](long long b, long long &q0, long long &q1) {
+        const long long r = b * 32 + lane;
+        q0 = __ldg(m.rowptr + (r < m.nrows ? r : m.nrows));
+        q1 = __ldg(m.rowptr + (r < m.nrows ? r + 1 : m.nrows));
+    };
+    long long b = (long long)blockIdx.x * BULK_WARPS + warp, q0 = 0, q1 = 0, n0 = 0, n1 = 0;
+    if (b < nb) bounds(b, q0, q1);
+    for (; b < nb; b += step, q0 = n0, q1 = n1) {
+        const long long a0 = __shfl_sync(full, q0, 0) & ~3ll;
+        const long long n = (__shfl_sync(full, q1, 31) - a0 + 3) & ~3ll;
+        bool staged = alive && n > 0 && n <= cap && a0 + n <= nnz;
+        if (staged && lane == 0) {
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                             smem_u32(bar)), "r"((unsigned)n * 12u) : "memory");
+            bulk_load(sv, m.values + a0, (unsigned)n * 8u, bar);
+            bulk_load(sc, m.colidx + a0, (unsigned)n * 4u, bar);
+        }
+        if (b + step < nb) bounds(b + step, n0, n1);   // while the copies run
+        const long long r = b * 32 + lane;
+        const double xr = TR && r < m.nrows ? __ldg(x + r) : 0.0;
+        const int len = (int)(q1 - q0);
+        const int most = (int)__reduce_max_sync(full, (unsigned)len);
+        if (staged) {
+            staged = alive = __all_sync(full, bar_wait(bar, phase));
+            if (staged) phase ^= 1u;
+        }
+        double acc = 0.0;
+        auto sum = [&](const double *v, const int *c) {
+            for (int k = 0; k < most; k += 4) {
+                double w[4], xv[4];
+                int cc[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const bool ok = k + j < len;
+                    cc[j] = ok ? c[k + j] : 0;
+                    w[j] = ok ? v[k + j] : 0.0;
+                }
+                if constexpr (TR) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (k + j < len) atomicAdd(y + cc[j], w[j] * xr);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) xv[j] = __ldg(x + cc[j]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        if (k + j < len) acc = fma(w[j], xv[j], acc);
+                }
+            }
+        };
+        if (staged) sum(sv + (q0 - a0), sc + (q0 - a0));
+        else sum(m.values + q0, m.colidx + q0);
+        if (!TR && r < m.nrows) y[r] = acc;
+        // the buffer's reads come before the copies that refill it
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+    }
+    if (!alive) (void)bar_wait(bar, phase);
+}
+
+// Runs the bulk kernel when the matrix suits it: rows short enough for 32 of
+// them to fit a buffer that leaves 20 warps or more per SM, enough rows to
+// give every warp two batches, arrays that 16-byte copies can start from.
+// Returns false, with nothing launched, otherwise.
+template <bool TR>
+bool spmv_csr_bulk(cudaStream_t st, const op2g_bcsr &m, long long nnz, const double *x, double *y,
+                   cudaError_t *e) {
+    *e = cudaSuccess;
+    if (nnz <= 0 || m.nrows < 1 || (uintptr_t)m.values % 16 || (uintptr_t)m.colidx % 16) return false;
+    const long long mean = (nnz + m.nrows - 1) / m.nrows;
+    if (mean > 20) return false;
+    const int cap = (int)((32 * mean + 32 + 63) / 64 * 64);
+    const int smem = cap * 12 * BULK_WARPS;
+    int per_sm = BULK_SMEM_PER_SM / (smem + 1024);   // 1 KB is the system's
+    if (per_sm > 16) per_sm = 16;
+    int dev = 0;
+    *e = cudaGetDevice(&dev);
+    if (*e != cudaSuccess) return true;
+    static thread_local int ready_on = -1, sms = 0;
+    if (dev != ready_on) {
+        *e = cudaFuncSetAttribute(k_spmv_csr_bulk<TR>,
+                                  cudaFuncAttributePreferredSharedMemoryCarveout, BULK_CARVEOUT);
+        if (*e != cudaSuccess) return true;
+        sms = sms_of_current();
+        ready_on = dev;
+    }
+    const long long ctas = (long long)per_sm * sms, nb = (m.nrows + 31) / 32;
+    if (nb < 2 * ctas * BULK_WARPS) return false;
+    k_spmv_csr_bulk<TR><<<(unsigned)ctas, 32 * BULK_WARPS, smem, st>>>(m, nnz, cap, x, y);
+    *e = cudaGetLastError();
+    return true;
+}
+
 // y += A^T x (y zeroed by the caller) for blocks up to 4 x 4; false when the
 // shape has no lane kernel.
 bool spmv_t_lane(cudaStream_t st, const op2g_bcsr &m, const double *x, double *y,
@@ -1760,6 +1918,11 @@ op2g_status op2g_mat_set_diagonal(const op2g_bcsr *m, const int32_t *rows, int64
 
 op2g_status op2g_mat_spmv(const op2g_bcsr *m, const double *x, double *y, int32_t transpose,
                           void *stream) {
+    return op2g_mat_spmv_sized(m, -1, x, y, transpose, stream);
+}
+
+op2g_status op2g_mat_spmv_sized(const op2g_bcsr *m, int64_t nblocks, const double *x, double *y,
+                                int32_t transpose, void *stream) {
     op2g_status s = check_bcsr(m);
     if (s != OP2G_OK) return s;
     const long long nr = m->nrows * m->rdim;
@@ -1767,6 +1930,12 @@ op2g_status op2g_mat_spmv(const op2g_bcsr *m, const double *x, double *y, int32_
     cudaStream_t st = (cudaStream_t)stream;
     const int r = m->rdim, c = m->cdim;
     cudaError_t te = cudaSuccess;
+    if (r == 1 && c == 1 && m->ncols <= INT_MAX &&
+        (transpose ? spmv_csr_bulk<true>(st, *m, nblocks, x, y, &te)
+                   : spmv_csr_bulk<false>(st, *m, nblocks, x, y, &te))) {
+        CK(te);
+        return OP2G_OK;
+    }
     if (transpose) {
         // blocks up to 4 x 4: the lane kernel, C atomics per block (128^3
         // tet mesh: CSR 0.110 ms, 3x3 0.596 ms, against 0.590 / 1.692 ms for

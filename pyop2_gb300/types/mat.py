@@ -777,8 +777,8 @@ class Mat(DataCarrier):
         b = self._bcsr()
         if transpose:
             y.tensor.zero_()
-        _lib.call("op2g_mat_spmv", ctypes.byref(b), x._device_ptr(), y._device_ptr(),
-                  1 if transpose else 0, device.stream_handle())
+        _lib.call("op2g_mat_spmv_sized", ctypes.byref(b), self._sparsity.nblocks, x._device_ptr(),
+                  y._device_ptr(), 1 if transpose else 0, device.stream_handle())
         y.mark_device_modified()
 
     def __str__(self):
