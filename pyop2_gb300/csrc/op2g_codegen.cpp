@@ -283,6 +283,7 @@ struct Gen {
     // cells' gathers and arithmetic can be interleaved by the compiler.
     bool guard_unpack = false;
     int cells_per_thread = 1;  // what the sweep loop was generated with
+    bool two_layers = false;   // op2g_run may take two layers per thread (layer_halves)
     // The variant for aligned direct arguments (aligned_direct_args).
     bool align_hints = false;
     // Elements a thread of a pure reduction loads together, 0 for other loops.
@@ -871,7 +872,7 @@ struct Gen {
     // the bottom ones of the next, which the next lane holds, go to the same
     // targets: they are added in registers and issued as one reduction, half
     // as many for the L2, which is what bounds a light loop.  8.4 M prisms,
-    // six floats each: 44 -> PAIR_F32 us, doubles 81 -> PAIR_F64 us.  Whether
+    // six doubles each: 81 -> 57 us (floats: 44 us either way).  Whether
     // the entries pair up is tested per column at run time.  Up to 12
     // components: larger packs come with kernels that the FP64 pipe bounds,
     // which the additions would only delay.
@@ -1124,7 +1125,10 @@ struct Gen {
         if (has_groups) warp = false;  // grouped packs scatter by atomics
         plan_shared(!extr && S.loop.scatter == OP2G_SCATTER_SHARED);
 
+        two_layers = layer_halves();
+
         // ----- the run function: a strided sweep of [start, end) plus reductions
+        if (two_layers) O << "template <int PARTS>\n";
         O << "__device__ __forceinline__ void op2g_run(const op2g_params_t &p, long long start, "
              "long long end, long long first, long long stride, int red_warps_) {\n";
         emit_global_init();
@@ -1137,7 +1141,9 @@ struct Gen {
             O << "  const int cs_ = lay_[0], ce_ = lay_[1] - 1;  // cellStart, cellEnd\n";
             emit_layer_extents("cs_", "ce_", "ls_", "le_", "  ");
             O << "  const long long nl_ = le_ > ls_ ? (long long)(le_ - ls_) : 0;\n";
-            O << "  const long long i0_ = start * nl_, i1_ = end * nl_;\n";
+            if (two_layers)
+                O << "  const long long sw_ = PARTS == 2 ? (nl_ + 1) >> 1 : nl_;  // swept\n";
+            O << "  const long long i0_ = start * " << swept() << ", i1_ = end * " << swept() << ";\n";
         } else {
             O << "  const long long i0_ = start, i1_ = end;\n";
         }
@@ -1208,11 +1214,11 @@ struct Gen {
         layer_pairs = step_layers;
         cell_pairs = !extr && cpt == 1;
         if (step_layers) {
-            O << "  const long long qs_ = nl_ ? op2g::div(stride, nl_) : 0;\n"
-              << "  const int rs_ = (int)(stride - qs_ * nl_);\n"
+            O << "  const long long qs_ = nl_ ? op2g::div(stride, " << swept() << ") : 0;\n"
+              << "  const int rs_ = (int)(stride - qs_ * " << swept() << ");\n"
               << "  const long long it0_ = i0_ + first + threadIdx.x;\n"
-              << "  long long it_ent = nl_ ? op2g::div(it0_, nl_) : 0;\n"
-              << "  int it_lay = (int)(it0_ - it_ent * nl_);\n";
+              << "  long long it_ent = nl_ ? op2g::div(it0_, " << swept() << ") : 0;\n"
+              << "  int it_lay = (int)(it0_ - it_ent * " << swept() << ");\n";
         }
         if (red_unroll) {
             O << "  for (long long base_ = i0_ + first; base_ < i1_; base_ += stride * " << red_unroll
@@ -1246,7 +1252,12 @@ struct Gen {
         } else {
             O << "  for (long long base_ = i0_ + first; base_ < i1_; base_ += stride) {\n";
             O << "    const long long it = base_ + threadIdx.x;\n";
-            O << "    const bool active = it < i1_;\n";
+            if (two_layers)
+                O << "#pragma unroll\n   for (int part_ = 0; part_ < PARTS; ++part_) {\n"
+                  << "    const int lay0_ = it_lay + part_ * (int)sw_;\n"
+                  << "    const bool active = it < i1_ && (part_ == 0 || lay0_ < nl_);\n";
+            else
+                O << "    const bool active = it < i1_;\n";
         }
         if (pf) {
             for (size_t m = 0; m < S.maps.size(); ++m)
@@ -1291,7 +1302,7 @@ struct Gen {
             bool combined = false;
             for (size_t a = 0; a < S.args.size(); ++a) combined = combined || deferred(a);
             if (step_layers && !S.loop.indexed && !combined) {
-                O << J << "if (it + stride < i1_) {\n";
+                O << J << "if (" << (two_layers ? "part_ == 0 && " : "") << "it + stride < i1_) {\n";
                 for (size_t m = 0; m < S.maps.size(); ++m)
                     if (rows[m])
                         O << J << "  asm volatile(\"prefetch.global.L2 [%0];\" :: \"l\"((const int *)p.ptr["
@@ -1299,7 +1310,7 @@ struct Gen {
                 O << J << "}\n";
             }
             if (step_layers) {
-                O << J << "const int layer = ls_ + it_lay;\n";
+                O << J << "const int layer = ls_ + " << (two_layers ? "lay0_" : "it_lay") << ";\n";
             } else {
                 O << J << "const long long it_ent = op2g::div(it, nl_);\n";
                 O << J << "const int layer = ls_ + (int)(it - it_ent * nl_);\n";
@@ -1397,9 +1408,10 @@ struct Gen {
             O << "    __syncthreads();\n";
             O << "    par_ ^= 1;\n";
         }
+        if (two_layers) O << "   }\n";  // parts of the column
         if (step_layers)
             O << "    it_ent += qs_;\n    it_lay += rs_;\n"
-              << "    if (it_lay >= nl_) { it_lay -= (int)nl_; ++it_ent; }\n";
+              << "    if (it_lay >= " << swept() << ") { it_lay -= (int)" << swept() << "; ++it_ent; }\n";
         if (cpt > 1 || red_unroll) O << "   }\n";  // cells of the step
         O << "  }\n";  // sweep loop
         guard_unpack = false;
@@ -1426,6 +1438,7 @@ struct Gen {
         // tables are sized for BS threads) the wrapper may be launched with
         // fewer threads per CTA than BS: a small iteration set is then
         // spread over more SMs (each SM issues FP64 at 2 per clock).
+        const char *one = two_layers ? "<1>" : "";
         const std::string bdim = any_shared ? std::to_string(BS) : std::string("blockDim.x");
         if (any_staged) {
             emit_staged_run();
@@ -1434,9 +1447,15 @@ struct Gen {
               << "  op2g_run_staged(p);\n}\n";
         } else {
             O << "extern \"C\" __global__ void __launch_bounds__(" << bounds
-              << ") op2g_wrap(const __grid_constant__ op2g_params_t p) {\n"
-              << "  op2g_run(p, p.start, p.end, (long long)blockIdx.x * " << bdim
-              << ", (long long)gridDim.x * " << bdim << ", " << red_warps(false) << ");\n}\n";
+              << ") op2g_wrap(const __grid_constant__ op2g_params_t p) {\n";
+            const std::string sweep = "(p, p.start, p.end, (long long)blockIdx.x * " + bdim +
+                                      ", (long long)gridDim.x * " + bdim + ", " +
+                                      std::to_string(red_warps(false)) + ");\n";
+            O << "  op2g_run" << one << sweep << "}\n";
+            if (two_layers)
+                O << "extern \"C\" __global__ void __launch_bounds__(" << BS
+                  << ") op2g_wrap_halves(const __grid_constant__ op2g_params_t p) {\n"
+                  << "  op2g_run<2>" << sweep << "}\n";
         }
         if (!any_shared && !any_staged) {
             // Balanced form for launches of a few CTAs per SM: CTA b takes the
@@ -1448,7 +1467,7 @@ struct Gen {
               << "  const long long c_ = (n_ + gridDim.x - 1) / gridDim.x;\n"
               << "  const long long s_ = p.start + (long long)blockIdx.x * c_;\n"
               << "  const long long e_ = s_ + c_ < p.end ? s_ + c_ : p.end;\n"
-              << "  if (s_ < e_) op2g_run(p, s_, e_, 0, (long long)blockDim.x, "
+              << "  if (s_ < e_) op2g_run" << one << "(p, s_, e_, 0, (long long)blockDim.x, "
               << red_warps(true) << ");\n}\n";
         }
         O << "extern \"C\" __global__ void __launch_bounds__(" << BS
@@ -1456,7 +1475,7 @@ struct Gen {
              "*__restrict__ work, long long nwork) {\n"
           << "  for (long long w = blockIdx.x; w < nwork; w += gridDim.x) {\n"
           << "    const op2g_params_t &p = P[work[3 * w]];\n"
-          << "    op2g_run(p, work[3 * w + 1], work[3 * w + 2], 0, " << BS << ", -1);\n"
+          << "    op2g_run" << one << "(p, work[3 * w + 1], work[3 * w + 2], 0, " << BS << ", -1);\n"
           << "  }\n}\n";
         return O.str();
     }
@@ -1483,6 +1502,30 @@ struct Gen {
         }
     }
 
+    // A thread of a light extruded loop over many cells takes two layers of a
+    // column, half the column apart (so that consecutive lanes still read
+    // consecutive layers): where they are, and the column's map rows, are
+    // worked out and loaded once for both.  8.4 M prisms out of memory, a mean
+    // of six floats 43 -> 37 us, six floats added to their nodes 55 -> 50.
+    // An entry of its own, launched over HALVES_CELLS cells in columns of
+    // HALVES_LAYERS or more: 262,144 prisms, six doubles added to their nodes,
+    // take 4.4 us one by one and 5.0 in twos, columns of 17 layers (2.1 M
+    // prisms) 17.4 and 19.3; one entry for both costs launches below the line
+    // 0.3 us.  Quarters of a column gain no more (means 2 us less, increments
+    // 2 us more).
+    bool layer_halves() const {
+        if (!S.loop.extruded || !S.loop.constant_layers || S.loop.scatter != OP2G_SCATTER_ATOMIC ||
+            S.loop.cells_per_thread > 1 || any_staged || has_groups ||
+            S.loop.iteration_region == OP2G_ON_BOTTOM || S.loop.iteration_region == OP2G_ON_TOP)
+            return false;
+        for (const ArgInfo &A : S.args)
+            if (A.d.kind == OP2G_ARG_DAT && A.d.map < 0 && A.d.access != OP2G_READ) return false;
+        return light_packs();
+    }
+
+    // Layers of a column that a sweep steps over.
+    const char *swept() const { return two_layers ? "sw_" : "nl_"; }
+
     // Scattered by the whole warp after the active block.
     bool deferred(size_t a) const {
         return (layer_pairs && combines_layers(a)) || (cell_pairs && combines_cells(a));
@@ -1499,7 +1542,8 @@ struct Gen {
         const std::string an = std::to_string(a);
         O << I << "{ " << T << " *d_ = (" << T << " *)p.ptr[" << A.slot << "];\n";
         O << I << "  const int lane_ = threadIdx.x & 31;\n";
-        O << I << "  const bool tx_ = pr" << an << "_ && lane_ < 31 && it_lay + 1 < nl_ && it + 1 < i1_;\n";
+        O << I << "  const bool tx_ = pr" << an << "_ && lane_ < 31 && it_lay + 1 < " << swept()
+          << (two_layers ? " && (part_ == 0 || lay0_ + 1 < nl_)" : "") << " && it + 1 < i1_;\n";
         O << I << "  if (__any_sync(0xffffffffu, pr" << an << "_)) {\n";
         O << I << "    const bool rx_ = pr" << an << "_ && lane_ > 0 && it_lay > 0;\n";
         O << "#pragma unroll\n" << I << "    for (int k = 0; k < " << h * D << "; ++k) {\n";
@@ -1967,6 +2011,7 @@ std::vector<std::pair<int, int>> aligned_direct_args(const Signature &S) {
 }
 
 int reduction_unroll(const Signature &S) { return Gen(S).reduction_unroll(); }
+bool layer_halves(const Signature &S) { return Gen(S).layer_halves(); }
 
 std::string generate_source(const Signature &S, int *cells_per_thread, bool align_hints) {
     Gen g(S);

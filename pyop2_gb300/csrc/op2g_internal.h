@@ -48,6 +48,10 @@ std::string generate_source(const Signature &S, int *cells_per_thread = nullptr,
                             bool align_hints = false);
 // Iterations a thread of a pure reduction loads together, 0 for other loops.
 int reduction_unroll(const Signature &S);
+// Whether there is an entry whose threads take two layers of a column at a
+// time, for HALVES_CELLS cells or more in columns of HALVES_LAYERS or more.
+bool layer_halves(const Signature &S);
+constexpr int HALVES_CELLS = 400000, HALVES_LAYERS = 32;
 // Direct Dat arguments whose rows are a multiple of 16 bytes, as (pointer
 // slot, row alignment in bytes: 16 or 32); empty for staged wrappers.
 std::vector<std::pair<int, int>> aligned_direct_args(const Signature &S);

@@ -215,10 +215,12 @@ constexpr int SMALL_CTA = 64;
 struct Loaded {
     CUmodule mod = nullptr;
     CUfunction f = nullptr, fb = nullptr, fc = nullptr;  // plain, batched, chunked
+    CUfunction fh = nullptr;  // two layers per thread (layer_halves)
     int regs = -1;
     int occ = 0;  // resident CTAs per SM
     int occ_small = 0;  // the same for CTAs of SMALL_CTA threads
     int occ_chunked = 0;  // resident CTAs per SM of the balanced entry
+    int occ_halves = 0;   // and of the entry for two layers per thread
     int sms = 0;
     // staged wrappers: dynamic shared memory the function is set up for, and
     // the resident CTAs per SM at the last size asked for
@@ -260,6 +262,10 @@ op2g_status load_module(const std::string &cubin, const char *fname, const char 
     if (!L.fc || D.OccupancyMaxActiveBlocksPerMultiprocessor(&L.occ_chunked, L.fc, bs, 0) !=
                      CUDA_SUCCESS)
         L.occ_chunked = L.occ;
+    if (D.ModuleGetFunction(&L.fh, L.mod, "op2g_wrap_halves") != CUDA_SUCCESS) L.fh = nullptr;
+    if (!L.fh || D.OccupancyMaxActiveBlocksPerMultiprocessor(&L.occ_halves, L.fh, bs, 0) !=
+                     CUDA_SUCCESS)
+        L.occ_halves = L.occ;
     if (bs > SMALL_CTA && D.OccupancyMaxActiveBlocksPerMultiprocessor(
                               &L.occ_small, L.f, SMALL_CTA, 0) != CUDA_SUCCESS)
         L.occ_small = 0;
@@ -642,20 +648,24 @@ op2g_status op2g_kernel_launch(op2g_kernel *k, const op2g_launch_desc *d, void *
     const int64_t items = (d->end - d->start) * (k->sig.loop.extruded && k->sig.loop.constant_layers &&
                                                  column_parallel(k->sig) ? per : 1);
     if (items <= 0) return OP2G_OK;
-    // a thread runs cells_per_thread iterations per sweep step: the grid is
-    // sized for the steps
-    const int64_t cpt = k->cells_per_thread > 1 ? k->cells_per_thread : 1;
+    // a thread runs cells_per_thread iterations per sweep step, or two layers
+    // of a column (unless the balanced entry runs): the grid is sized for the
+    // steps
+    const bool halves = L->fh && per >= HALVES_LAYERS && items >= HALVES_CELLS &&
+                        (d->grid != 0 || items >= 8ll * L->sms * k->sig.block_size);
+    const int64_t cpt = halves ? 2 : k->cells_per_thread > 1 ? k->cells_per_thread : 1;
     int32_t grid = 0, bs = 0, chunked = 0;
     op2g_launch_shape((items + cpt - 1) / cpt, (d->end - d->start + cpt - 1) / cpt,
-                      k->sig.block_size, L->sms, L->occ, d->grid, L->fc != nullptr, &grid, &bs,
-                      &chunked);
+                      k->sig.block_size, L->sms, halves ? L->occ_halves : L->occ, d->grid,
+                      L->fc != nullptr, &grid, &bs, &chunked);
     // A pure reduction runs one resident wave: its threads keep accumulators,
     // and fewer of them settle sooner and reduce into fewer atomics.
     if (d->grid == 0 && k->reduction && !chunked)
         grid = (int32_t)std::min<int64_t>(grid, (int64_t)L->occ * L->sms);
     else if (d->grid == 0) refine_shape(*L, k->sig, (items + cpt - 1) / cpt, &grid, &bs, &chunked);
     void *params[] = {buf};
-    return launch(chunked ? L->fc : L->f, (unsigned)grid, (unsigned)bs, params, stream);
+    return launch(chunked ? L->fc : halves ? L->fh : L->f, (unsigned)grid, (unsigned)bs, params,
+                  stream);
 }
 
 void op2g_launch_shape(int64_t items, int64_t entities, int32_t block_size, int32_t sms,
